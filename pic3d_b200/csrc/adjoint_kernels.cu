@@ -1149,7 +1149,7 @@ void adjoint_record_hook(pic_ctx *c) {
     for (int k = 0; k < 2; ++k) {
         Species &s = c->sp[k];
         if (c->tile <= 0 || s.n_host == 0 || !s.sorted || !A->toffs[k]) continue;
-        const long long kpt = (long long)c->tile * c->tile * c->tile * kOctants;
+        const long long kpt = c->keys_per_tile;
         tile_bounds_kernel<<<(ntiles + 256) / 256, 256, 0, c->stream>>>(s.offs, kpt, ntiles, A->toffs[k]);
         toff_part[k] = (int)parts.size();
         parts.push_back({A->toffs[k], (size_t)(ntiles + 1) * sizeof(unsigned)});

@@ -32,8 +32,8 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs<real> a) {
             continue;
         }
         const PmSrc<real> pm{a.px, a.py, a.pz, a.w, p};
-        push_body<real, P, SPIN, true>(a, p, o, pm, fv, acc, [&](const int (&cn)[3]) {
-            if (a.idx_pairs) vis_note(a.vsink, a.g, (int)p, a.idx[2 * t + 1], cn);
+        push_body<real, P, SPIN, true>(a, p, o, pm, fv, acc, [&](const int (&cn)[3], const int (&nn)[3]) {
+            if (a.idx_pairs) vis_note(a.vsink, a.g, (int)p, a.idx[2 * t + 1], cn, nn);
         });
     }
 }
@@ -117,6 +117,7 @@ struct RemoveArgs {
     int *holes, *movers;
     const double *x, *y, *z;
     const int *cell;
+    const float *ox, *oy, *oz;
 };
 
 __device__ __forceinline__ bool is_dead(const RemoveArgs &a, long long i) {
@@ -176,10 +177,14 @@ struct MoveArgs {
     long long keys_per_tile;
 };
 
-// the cell the next push's decode will see (as push_body reports it)
-__device__ __forceinline__ void current_cell(const RemoveArgs &a, long long i, int (&c)[3]) {
+// the cell and the node the next push's decode will see (as push_move
+// reports them)
+__device__ __forceinline__ void current_cell(const RemoveArgs &a, long long i, int (&c)[3], int (&nd)[3]) {
     if (a.fp32) {
         a.cp.unpack(a.cell[i], c[0], c[1], c[2]);
+        const float o[3] = {a.ox[i], a.oy[i], a.oz[i]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) nd[d] = c[d] + (o[d] >= 0.5f ? 1 : 0);
         return;
     }
     const double v0[3] = {a.x[i], a.y[i], a.z[i]};
@@ -192,6 +197,7 @@ __device__ __forceinline__ void current_cell(const RemoveArgs &a, long long i, i
         }
         const double xc = v - (double)(1 - a.g.mem);
         c[d] = xc >= 0.0 ? (int)xc - (a.g.mem - 1) : -1;
+        nd[d] = xc >= 0.0 ? (int)(xc + 0.5) - (a.g.mem - 1) : -1;
     }
 }
 
@@ -219,10 +225,10 @@ __global__ void apply_moves_kernel(MoveArgs a) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) mv(a.i[k], dst, src);
     if (a.vsink.raw) {
-        int c[3];
-        current_cell(a.at, src, c);
+        int c[3], nd[3];
+        current_cell(a.at, src, c, nd);
         const int nt = a.vsink.nt[0] * a.vsink.nt[1] * a.vsink.nt[2];
-        vis_note(a.vsink, a.at.g, dst, home_tile(a.offs, a.keys_per_tile, nt, dst), c);
+        vis_note(a.vsink, a.at.g, dst, home_tile(a.offs, a.keys_per_tile, nt, dst), c, nd);
     }
 }
 
@@ -277,6 +283,7 @@ void launch_remove(pic_ctx *c, int kind) {
     int cu = s.cur;
     a.x = s.a.x[cu]; a.y = s.a.y[cu]; a.z = s.a.z[cu];
     a.cell = s.a.cell[cu];
+    a.ox = s.a.ox[cu]; a.oy = s.a.oy[cu]; a.oz = s.a.oz[cu];
     cudaMemsetAsync(c->d_scratch_ll, 0, 3 * sizeof(long long), c->stream);
     unsigned blocks = (unsigned)((n + 255) / 256);
     count_dead_kernel<<<blocks, 256, 0, c->stream>>>(a);
@@ -307,7 +314,7 @@ void launch_remove(pic_ctx *c, int kind) {
         m.vsink = vis_sink_of(c, s);
         m.at = a;
         m.offs = s.offs;
-        m.keys_per_tile = (long long)c->tile * c->tile * c->tile * kOctants;
+        m.keys_per_tile = c->keys_per_tile;
         vis_drop_kernel<<<148 * 4, 256, 0, c->stream>>>(a, s.vraw, s.vs, s.vcap);
     }
     apply_moves_kernel<<<blocks, 256, 0, c->stream>>>(m);

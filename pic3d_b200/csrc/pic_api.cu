@@ -532,10 +532,16 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     // of the reverse sweep (each sort's permutation goes on the tape).
     c->sort_interval = p.sort_interval > 0 ? p.sort_interval : (p.adjoint ? 1 : 4);
     if (c->tile > 0) {
-        for (int d = 0; d < 3; ++d) c->ntile[d] = (n[d] + c->tile - 1) / c->tile;
-        c->nkeys = (long long)c->ntile[0] * c->ntile[1] * c->ntile[2] * kOctants * c->tile * c->tile * c->tile;
-        if (c->nkeys >= (1ll << 31)) return bad("too many sort keys");
-        if (tile_smem_bytes(c) > 227 * 1024) return bad("tile too large for shared memory");
+        c->node_tiles = node_tiles_for(c->tile, p.adjoint != 0, c->order);
+        // cells 0 .. n-1, or nodes 0 .. n
+        for (int d = 0; d < 3; ++d) c->ntile[d] = (n[d] + (c->node_tiles ? 1 : 0) + c->tile - 1) / c->tile;
+        c->keys_per_tile = (long long)c->tile * c->tile * c->tile * (c->node_tiles ? 1 : kOctants);
+        c->nkeys = (long long)c->ntile[0] * c->ntile[1] * c->ntile[2] * c->keys_per_tile;
+        // (the limit of tiles of cells, whichever kind is used)
+        long long cell_keys = kOctants;
+        for (int d = 0; d < 3; ++d) cell_keys *= (long long)((n[d] + c->tile - 1) / c->tile) * c->tile;
+        if (cell_keys >= (1ll << 31) || c->nkeys >= (1ll << 31)) return bad("too many sort keys");
+        if ((c->node_tiles ? node_tile_smem_bytes(c) : tile_smem_bytes(c)) > 227 * 1024) return bad("tile too large for shared memory");
     }
     c->device = device;
     cudaError_t e = cudaSetDevice(device);

@@ -125,6 +125,7 @@ struct VisSink {
     VisState *vs;
     long long cap;               // triples
     int T, nt[3];
+    int nodes;                   // 1: tiles hold nodes (pic_ctx::node_tiles), 0: cells
 };
 
 struct Species {
@@ -217,9 +218,14 @@ struct pic_ctx {
     int64_t pin_records = 0;
     cudaEvent_t pin_ev[2] = {nullptr, nullptr};
     // tiling / sorting
-    int tile = 0;                        // tile edge in cells (0: global-memory kernel only)
+    int tile = 0;                        // tile edge in cells (or nodes) (0: global-memory kernel only)
     int ntile[3] = {0, 0, 0};
-    long long nkeys = 0;                 // ntiles * kOctants * tile^3
+    // Tiles of nodes (particles by their primal stencil index, sorted by node
+    // within the tile) instead of tiles of cells (sorted by half-cell octant,
+    // then cell): what the matrix deposit of tile_mma_kernels.cu needs
+    bool node_tiles = false;
+    long long keys_per_tile = 0;         // tile^3 (nodes) or kOctants * tile^3 (cells)
+    long long nkeys = 0;                 // ntiles * keys_per_tile
     unsigned *d_hist = nullptr;          // nkeys + 1
     unsigned *d_blocksums = nullptr;
     unsigned long long *d_nstrag = nullptr;   // straggler counts, one per species

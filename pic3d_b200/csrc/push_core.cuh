@@ -16,11 +16,16 @@ namespace pic {
 // x = n, wrapped only at the next push) cannot be binned: the next push
 // falls back to the global kernel for particles away from home.  Outside on
 // a non-periodic axis the particle is removed before the next push.
+// Where tiles hold nodes (VisSink::nodes) the particle's primal index takes
+// the place of its cell: 0 .. n per axis, so that x = n has a tile too.
 // `here`, `lo`: a tile the cell is likely in (the pushing CTA's) and its
 // first cell per axis (here < 0: none), which spares the divisions.
-__device__ __forceinline__ void vis_note(const VisSink &v, const Geom &g, int p, int home, const int (&cell)[3],
-                                         int here = -1, const int *lo = nullptr) {
+__device__ __forceinline__ void vis_note(const VisSink &v, const Geom &g, int p, int home, const int (&at_cell)[3],
+                                         const int (&at_node)[3], int here = -1, const int *lo = nullptr) {
     if (!v.raw) return;
+    int cell[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) cell[d] = v.nodes ? at_node[d] : at_cell[d];
     int t = -1;
     if (here >= 0) {
         bool in_here = true;
@@ -33,7 +38,7 @@ __device__ __forceinline__ void vis_note(const VisSink &v, const Geom &g, int p,
         bool in = true, per_out = false;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const bool o = cell[d] < 0 || cell[d] >= g.n[d];
+            const bool o = cell[d] < 0 || cell[d] >= g.n[d] + v.nodes;
             in = in && !o;
             per_out = per_out || (o && g.per[d]);
         }
@@ -81,7 +86,6 @@ struct PushArgs {
     real qm;                 // charge / mass * dt_half (particle.cpp:271)
     real charge;
     real dt_d[3];            // dt / dx, dt / dy, dt / dz
-    double dt_s, dxs[3];     // dt and dx, dy, dz
     real d_dt[3];            // dx / dt, dy / dt, dz / dt (particle.cpp:423-425)
     double E_schwinger, dt_half_d, charge_d, mass_d;
     int electron;            // spin precession applies to this species (particle.cpp:318-319)
@@ -544,18 +548,38 @@ __device__ __forceinline__ void decode_old(const PushArgs<real> &a, long long p,
     }
 }
 
-// Everything after the position decode: gather, Boris, move, deposit,
-// store, spin.  fv: the six field views; jv: view for the current arrays
-// (jx..rho share its strides).
+// 1 / sqrt(x), x >= 1: the library's FP64 function (1 ulp); in FP32 the
+// hardware approximation (2 ulp) with one Newton step (x = inf, where the
+// step is not a number, gives 0 as the division by gamma did).  A square root
+// and the divisions by it cost three times as many instructions.
+__device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
+__device__ __forceinline__ float inv_sqrt(float x) {
+    const float y = rsqrtf(x);
+    return y > 0.0f ? fmaf(0.5f * y, fmaf(-x * y, y, 1.0f), y) : y;
+}
+
+// A particle's move as its deposit needs it: old and new primal index, the
+// old primal offset d0, and the new primal offset (FP64) or the move in cells
+// (FP32) in dm.
+template <typename real>
+struct Moved {
+    int i1[3], i2[3];
+    real d0[3], dm[3];
+    real qw;
+    bool moved;   // changed position (one at rest adds no current, only rho)
+};
+
+// Everything after the position decode and before the deposit: gather,
+// Boris, move, store, spin.  fv: the six field views.
 // Returns false when the particle was skipped (non-finite momentum or a move
-// over a cell: status set, nothing stored).  The new state is stored before
-// the deposit (fewer values live through its loops); note(cnew) is called
-// then with the new cell as the next push's decode will see it.
-template <typename real, int P, bool SPIN, bool LDG, class Acc, class Note>
-__device__ __forceinline__ bool push_body(const PushArgs<real> &a, long long p, const OldPos<real> &o,
-                                          const PmSrc<real> &pm, const View<const real> (&fv)[6], const Acc &acc,
-                                          Note &&note) {
-    int cnew[3];
+// over a cell: status set, nothing stored).  note(cell, node) is called with
+// the new cell and the new primal index (domain coordinates) as the next
+// push's decode will see them.
+template <typename real, int P, bool SPIN, bool LDG, class Note>
+__device__ __forceinline__ bool push_move(const PushArgs<real> &a, long long p, const OldPos<real> &o,
+                                          const PmSrc<real> &pm, const View<const real> (&fv)[6], Note &&note,
+                                          Moved<real> &mv) {
+    int cnew[3], nnew[3];
     constexpr bool F64 = cuda::std::is_same<real, double>::value;
     constexpr int H = P / 2;
     const Geom &g = a.g;
@@ -578,8 +602,8 @@ __device__ __forceinline__ bool push_body(const PushArgs<real> &a, long long p, 
     real ex_p = e0 * qm, ey_p = e1 * qm, ez_p = e2 * qm;
     real bx_p = b0 * qm, by_p = b1 * qm, bz_p = b2 * qm;
     real px1 = pm.px[pm.i] + ex_p, py1 = pm.py[pm.i] + ey_p, pz1 = pm.pz[pm.i] + ez_p;
-    real gm1 = sqrt(real(1) + (px1 * px1 + py1 * py1 + pz1 * pz1));
-    real tx = bx_p / gm1, ty = by_p / gm1, tz = bz_p / gm1;
+    const real ig1 = inv_sqrt(real(1) + (px1 * px1 + py1 * py1 + pz1 * pz1));
+    real tx = bx_p * ig1, ty = by_p * ig1, tz = bz_p * ig1;
     real tt = real(2) / (real(1) + tx * tx + ty * ty + tz * tz);
     real sx = tx * tt, sy = ty * tt, sz = tz * tt;
     real px2 = px1 + (py1 * tz - pz1 * ty);
@@ -588,32 +612,31 @@ __device__ __forceinline__ bool push_body(const PushArgs<real> &a, long long p, 
     real pxn = px1 + (py2 * sz - pz2 * sy) + ex_p;
     real pyn = py1 + (pz2 * sx - px2 * sz) + ey_p;
     real pzn = pz1 + (px2 * sy - py2 * sx) + ez_p;
-    real gam = sqrt(real(1) + (pxn * pxn + pyn * pyn + pzn * pzn));
+    const real g2 = real(1) + (pxn * pxn + pyn * pyn + pzn * pzn);
+    const real ig = inv_sqrt(g2);
     // move in cell units (particle.cpp:313-315)
     int i2[3];
-    double d2[3];   // FP64: new primal offsets
     double xn[3];
     int cn[3];
     real on[3];
-    real disp[3];   // FP32: the move in cells
     if constexpr (F64) {
-        xn[0] = o.xd[0] + (double)pxn / (double)gam * a.dt_s / a.dxs[0];
-        xn[1] = o.xd[1] + (double)pyn / (double)gam * a.dt_s / a.dxs[1];
-        xn[2] = o.xd[2] + (double)pzn / (double)gam * a.dt_s / a.dxs[2];
+        xn[0] = o.xd[0] + pxn * ig * a.dt_d[0];
+        xn[1] = o.xd[1] + pyn * ig * a.dt_d[1];
+        xn[2] = o.xd[2] + pzn * ig * a.dt_d[2];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             double xc = xn[d] - (double)(1 - g.mem);
             i2[d] = (int)(xc + 0.5);
-            d2[d] = xc - (double)i2[d];
+            mv.dm[d] = xc - (double)i2[d];
         }
     } else {
-        disp[0] = pxn / gam * a.dt_d[0];
-        disp[1] = pyn / gam * a.dt_d[1];
-        disp[2] = pzn / gam * a.dt_d[2];
+        mv.dm[0] = pxn * ig * a.dt_d[0];
+        mv.dm[1] = pyn * ig * a.dt_d[1];
+        mv.dm[2] = pzn * ig * a.dt_d[2];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             // stored position: cell + FP32 offset in [0, 1)
-            real q = o.oo[d] + disp[d];
+            real q = o.oo[d] + mv.dm[d];
             int s = 0;
             if (q >= real(1)) { q -= real(1); s = 1; }
             else if (q < real(0)) {
@@ -651,41 +674,36 @@ __device__ __forceinline__ bool push_body(const PushArgs<real> &a, long long p, 
             }
             const double xc = v - (double)(1 - g.mem);
             cnew[d] = xc >= 0.0 ? (int)xc - (g.mem - 1) : -1;
+            nnew[d] = xc >= 0.0 ? (int)(xc + 0.5) - (g.mem - 1) : -1;
         }
     } else {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             if (g.per[d]) cn[d] = cn[d] < 0 ? cn[d] + g.n[d] : (cn[d] >= g.n[d] ? cn[d] - g.n[d] : cn[d]);
             cnew[d] = cn[d];
+            nnew[d] = cn[d] + (on[d] >= real(0.5) ? 1 : 0);
         }
         a.c1[p] = a.cp.pack(cn[0], cn[1], cn[2]);
         a.ox1[p] = on[0];
         a.oy1[p] = on[1];
         a.oz1[p] = on[2];
     }
-    note(cnew);
-    const real qw = a.charge * pm.w[pm.i];
-    Axis1D<real, P> ax[3];
-    bool moved = false;
-    if constexpr (F64) {
+    note(cnew, nnew);
+    mv.qw = a.charge * pm.w[pm.i];
+    mv.moved = false;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            axis_from_offsets<real, P>(o.ip[d], o.dp[d], i2[d], d2[d], ax[d]);
-            moved = moved || i2[d] != o.ip[d] || d2[d] != o.dp[d];
-        }
-    } else {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            axis_from_move<P>(o.ip[d], o.dp[d], disp[d], i2[d], ax[d]);
-            moved = moved || disp[d] != real(0);
-        }
+    for (int d = 0; d < 3; ++d) {
+        mv.i1[d] = o.ip[d];
+        mv.i2[d] = i2[d];
+        mv.d0[d] = o.dp[d];
+        if constexpr (F64) mv.moved = mv.moved || i2[d] != o.ip[d] || mv.dm[d] != o.dp[d];
+        else mv.moved = mv.moved || mv.dm[d] != real(0);
     }
-    deposit<real, P>(acc, a.d_dt, ax, moved, qw);
     // electron spin precession (particle.cpp:318-368)
     if constexpr (SPIN) {
         if (a.electron) {
             double exq = e0, eyq = e1, ezq = e2, bxq = b0, byq = b1, bzq = b2;
-            double g0 = gam;
+            double g0 = sqrt((double)g2);
             double vx = (double)pxn / g0, vy = (double)pyn / g0, vz = (double)pzn / g0;
             double pe = vx * exq + vy * eyq + vz * ezq;
             double fx = exq + vy * bzq - vz * byq;
@@ -714,6 +732,24 @@ __device__ __forceinline__ bool push_body(const PushArgs<real> &a, long long p, 
             a.sz[p] = (real)(s_z + (rx * uy - ry * ux) * t2);
         }
     }
+    return true;
+}
+
+// push_move, then the particle's deposit into acc.  The new state is stored
+// before the deposit (fewer values live through its loops).
+template <typename real, int P, bool SPIN, bool LDG, class Acc, class Note>
+__device__ __forceinline__ bool push_body(const PushArgs<real> &a, long long p, const OldPos<real> &o,
+                                          const PmSrc<real> &pm, const View<const real> (&fv)[6], const Acc &acc,
+                                          Note &&note) {
+    Moved<real> mv;
+    if (!push_move<real, P, SPIN, LDG>(a, p, o, pm, fv, note, mv)) return false;
+    Axis1D<real, P> ax[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        if constexpr (sizeof(real) == 8) axis_from_offsets<real, P>(mv.i1[d], mv.d0[d], mv.i2[d], mv.dm[d], ax[d]);
+        else axis_from_move<P>(mv.i1[d], mv.d0[d], mv.dm[d], mv.i2[d], ax[d]);
+    }
+    deposit<real, P>(acc, a.d_dt, ax, mv.moved, mv.qw);
     return true;
 }
 
@@ -769,7 +805,6 @@ inline PushArgs<real> make_push_args(pic_ctx *c, int kind) {
     a.qm = (real)(p.charge[kind] / p.mass[kind] * p.dt_half);
     a.charge = (real)p.charge[kind];
     a.dt_d[0] = (real)(p.dt / p.dx); a.dt_d[1] = (real)(p.dt / p.dy); a.dt_d[2] = (real)(p.dt / p.dz);
-    a.dt_s = p.dt; a.dxs[0] = p.dx; a.dxs[1] = p.dy; a.dxs[2] = p.dz;
     a.d_dt[0] = (real)(p.dx / p.dt); a.d_dt[1] = (real)(p.dy / p.dt); a.d_dt[2] = (real)(p.dz / p.dt);
     a.E_schwinger = p.E_schwinger; a.dt_half_d = p.dt_half; a.charge_d = p.charge[kind]; a.mass_d = p.mass[kind];
     a.electron = spin_active(c, kind) ? 1 : 0;

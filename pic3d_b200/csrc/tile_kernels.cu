@@ -21,21 +21,9 @@
 //
 // The counting sort (key histogram, exclusive scan, scatter into the second
 // set of arrays) runs every `sort_interval` pushes and after an upload.
-#include <algorithm>
-#include <cmath>
-
-#include "pic_kernels.cuh"
-#include "push_core.cuh"
+#include "tile_common.cuh"
 
 namespace pic {
-
-struct TileGeom {
-    int T, nt[3];
-    long long nkeys;
-    int GE, DE, nacc;
-    // padded shared-memory strides: row gsy/dsy, plane gsz/dsz, array gsize/dsize
-    int gsy, gsz, gsize, dsy, dsz, dsize;
-};
 
 // Row and plane strides of a shared-memory box of extent e for tile edge T.
 // Lanes of a warp take 32 consecutive cells of the tile (cell index
@@ -48,24 +36,27 @@ static inline void padded_strides(int e, int T, int &sy, int &sz) {
     sz = padded_plane(e, T);
 }
 
-template <int P>
-__host__ __device__ constexpr int gather_extent(int T) { return T + 2 * (P / 2) + 1; }
-template <int P>
-__host__ __device__ constexpr int deposit_extent(int T) { return T + 2 * (P / 2) + 3; }
-
 // Sort key of a particle in cell (cx, cy, cz) whose position in the cell
 // lies in half-cell octant `oct` (bit d set: offset >= 1/2 along axis d, so
-// its primal stencil index is the cell's plus one along d): tile, then
-// octant, then cell within the tile.
-__device__ __forceinline__ int cell_key(const TileGeom &t, int cx, int cy, int cz, int oct) {
+// its primal stencil index, its node, is the cell's plus one along d).
+// Tiles of cells: tile, then octant, then cell within the tile.  Tiles of
+// nodes: tile, then node within the tile, x fastest, so that consecutive
+// particles share the y and z of their stencils.
+__device__ __forceinline__ int tile_key(const TileGeom &t, const int (&cell)[3], int oct) {
     const int T = t.T;
-    int tx = cx / T, ty = cy / T, tz = cz / T;
-    int lx = cx - tx * T, ly = cy - ty * T, lz = cz - tz * T;
-    return ((((tz * t.nt[1] + ty) * t.nt[0] + tx) * kOctants + oct) * T + lz) * T * T + ly * T + lx;
+    int q[3], l[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int c = cell[d] + (t.nodes ? (oct >> d) & 1 : 0);
+        q[d] = c / T;
+        l[d] = c - q[d] * T;
+    }
+    const int tile = (q[2] * t.nt[1] + q[1]) * t.nt[0] + q[0];
+    return ((t.nodes ? tile : tile * kOctants + oct) * T + l[2]) * T * T + l[1] * T + l[0];
 }
 
-// cell of a particle for sorting (FP64: periodic wrap as the next push
-// will apply it; clamped into the domain)
+// sort key of particle i (FP64: periodic wrap as the next push will apply
+// it; cell clamped into the domain)
 __device__ __forceinline__ int particle_key(const Geom &g, const TileGeom &t, const CellPack &cp, int fp32,
                                             const double *x, const double *y, const double *z, const int *cell,
                                             const float *ox, const float *oy, const float *oz, long long i) {
@@ -88,7 +79,7 @@ __device__ __forceinline__ int particle_key(const Geom &g, const TileGeom &t, co
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d) c[d] = min(max(c[d], 0), g.n[d] - 1);
-    return cell_key(t, c[0], c[1], c[2], oct);
+    return tile_key(t, c, oct);
 }
 
 // ---------------------------------------------------------------------------
@@ -328,6 +319,7 @@ static TileGeom tile_geom(const pic_ctx *c) {
     t.T = c->tile;
     for (int d = 0; d < 3; ++d) t.nt[d] = c->ntile[d];
     t.nkeys = c->nkeys;
+    t.nodes = c->node_tiles ? 1 : 0;
     return t;
 }
 
@@ -440,50 +432,6 @@ static void prepare_push(pic_ctx *c, int mask) {
 
 // ---------------------------------------------------------------------------
 // the tile kernel
-
-// limbs of the shared-memory fixed-point accumulators
-template <typename real>
-constexpr int limbs() { return sizeof(real) == 8 ? 3 : 2; }
-// |value * scale| stays below 2^fixed_bits: with at most kMaxTileParticles
-// additions per point the limb sums fit in 32 bits and the reassembled
-// total in 64 bits (FixedAcc)
-constexpr int kMaxTileParticles = 16383;
-
-// Asynchronous global -> shared copies (cp.async): a CTA issues every copy
-// of a batch without waiting on any, then waits once.  src_bytes 0 fills the
-// destination with zeros and reads nothing.
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void *dst, const void *src, int src_bytes = BYTES) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(BYTES), "r"(src_bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-// word offset (from the accumulators) of the particle input buffers: after
-// the five accumulators, rounded up to 16 bytes
-__host__ __device__ constexpr int particle_buffer_offset(int acc_words) { return (acc_words + 3) & ~3; }
-
-template <typename real>
-struct TileArgs {
-    PushArgs<real> sp[2];
-    const unsigned *offs[2];
-    int active[2];
-    TileGeom t;
-    real *ring[5];
-    const real *field[6];
-    real scale[4];          // jx, jy, jz, rho
-    double inv_scale[4];
-    int *strag[2];          // (index, home tile) of particles left for the global kernel
-    unsigned long long *nstrag;
-    // visitor lists of this push (vis_off null: none) and the recording of
-    // the next push's (vsink.raw null: off)
-    const int *vis[2];
-    const unsigned *vis_off[2];
-    const VisState *vs[2];
-    VisSink vsink[2];
-};
 
 // Threads per CTA of an ordinary step (the kernel's launch bounds ask for
 // two CTAs per SM at 256 threads, one at 512: 128 registers either way).
@@ -654,8 +602,8 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) tile_push_kernel(Tile
                     constexpr int mo = PartIn<real>::kPos;   // momenta, then weight
                     const real *pr = reinterpret_cast<const real *>(sp_in + slot * KW * 32);
                     const PmSrc<real> pm{pr + mo * 32, pr + (mo + 1) * 32, pr + (mo + 2) * 32, pr + (mo + 3) * 32, lane};
-                    push_body<real, P, SPIN, false>(a, p, o, pm, fs, af, [&](const int (&cn)[3]) {
-                        vis_note(ta.vsink[k], g, (int)p, home, cn, tile, t0);
+                    push_body<real, P, SPIN, false>(a, p, o, pm, fs, af, [&](const int (&cn)[3], const int (&nn)[3]) {
+                        vis_note(ta.vsink[k], g, (int)p, home, cn, nn, tile, t0);
                     });
                 } else if (!inside && idx < mh && vvalid[k]) {
                     // away from home: pushed from the visitor list of the tile it is in
@@ -739,45 +687,14 @@ VisSink vis_sink_of(const pic_ctx *c, const Species &s) {
     v.vs = s.vs;
     v.cap = s.vcap;
     v.T = c->tile;
+    v.nodes = c->node_tiles ? 1 : 0;
     for (int d = 0; d < 3; ++d) v.nt[d] = c->ntile[d];
     return v;
 }
 
 template <typename real, int P, bool SPIN>
 static void tile_push_t(pic_ctx *c, int mask) {
-    TileArgs<real> ta{};
-    double qw_max = 0.0;
-    for (int k = 0; k < 2; ++k) {
-        ta.sp[k] = make_push_args<real>(c, k);
-        ta.offs[k] = c->sp[k].offs;
-        ta.active[k] = ((mask >> k) & 1) && c->sp[k].n_host > 0;
-        if (ta.active[k]) qw_max = std::max(qw_max, std::fabs(c->p.charge[k]) * c->sp[k].max_abs_w);
-    }
-    ta.t = tile_layout(c);
-    for (int k = 0; k < 5; ++k) ta.ring[k] = (real *)c->ring[k];
-    for (int k = 0; k < 6; ++k) ta.field[k] = (const real *)c->field[k];
-    // one contribution is at most |q w| d/dt (J: the running sum of ds and the
-    // Esirkepov weight are both within [-1, 1]) or |q w| smax^3 (rho, smax the
-    // largest shape weight: 3/4 at 2nd order, 115/192 at 4th)
-    const double dmax = std::max(c->p.dx, std::max(c->p.dy, c->p.dz));
-    const double lim = std::ldexp(1.0, fixed_bits<real>());
-    const double smax = P == 3 ? 0.75 : 115.0 / 192.0;
-    const double bj = 1.01 * qw_max * dmax / c->p.dt, br = 1.01 * qw_max * smax * smax * smax;
-    for (int k = 0; k < 4; ++k) {
-        double b = k < 3 ? bj : br;
-        double s = b > 0.0 ? lim / b : 1.0;
-        ta.scale[k] = (real)s;
-        ta.inv_scale[k] = 1.0 / (double)ta.scale[k];
-    }
-    for (int k = 0; k < 2; ++k) {
-        Species &s = c->sp[k];
-        ta.strag[k] = s.strag;
-        ta.vis[k] = s.vis;
-        ta.vis_off[k] = s.vis_off;
-        ta.vs[k] = s.vs;
-        ta.vsink[k] = vis_sink_of(c, s);
-    }
-    ta.nstrag = c->d_nstrag;
+    const TileArgs<real> ta = make_tile_args<real, P>(c, mask, tile_layout(c));
     cudaMemsetAsync(c->d_nstrag, 0, 2 * sizeof(unsigned long long), c->stream);
     size_t smem = tile_smem_bytes(c);
     const int ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
@@ -828,7 +745,9 @@ void launch_tile_push(pic_ctx *c, int mask) {
     prepare_push(c, mask);
     bool spin = ((mask & 1) && spin_active(c, 0)) || ((mask & 2) && spin_active(c, 1));
     prof_begin(c, "tile_push_gather_deposit");
-    if (c->fp32) {
+    if (c->node_tiles) {
+        launch_node_tile_kernel(c, mask, spin);
+    } else if (c->fp32) {
         if (c->order == 2) spin ? tile_push_t<float, 3, true>(c, mask) : tile_push_t<float, 3, false>(c, mask);
         else spin ? tile_push_t<float, 5, true>(c, mask) : tile_push_t<float, 5, false>(c, mask);
     } else {
