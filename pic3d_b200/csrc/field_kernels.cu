@@ -4,11 +4,13 @@
 // All are HBM-bound stencils or face/shell copies.  The Yee updates run one
 // thread per physical cell with x fastest (coalesced); neighbour reads come
 // through L1/L2.  The periodic halo exchange of the reference
-// (src/mpi_utils.cpp:9-60) and the ghost accumulation of the currents
-// (src/mpi_utils.cpp:232-417) become single-launch shell kernels: every
-// ghost point pulls its periodic image, every boundary point sums and then
-// broadcasts its images; each point has exactly one owning thread, so no
-// atomics are needed.
+// (src/mpi_utils.cpp:9-60) is part of each update: a cell's thread stores its
+// value to the cell's periodic images.  The ghost accumulation of the
+// currents (src/mpi_utils.cpp:232-417) is a shell pass: every boundary point
+// sums and then broadcasts its images.  Each point has exactly one owning
+// thread, so no atomics are needed.
+#include <algorithm>
+
 #include "pic_kernels.cuh"
 #include "push_core.cuh"
 
@@ -38,52 +40,109 @@ Geom make_geom(const PicParams &p) {
 
 // ---------------------------------------------------------------------------
 // Yee half-updates over the physical cells (src/field.cpp:59-67 and :74-82)
+// with the periodic ghost fill of the updated arrays: the thread of a point
+// stores its value to the point's periodic images too (none of them is read
+// by the same launch: E reads B and its own E, and the other way round).
+//
+// What bounds them: HBM on large grids (256 x 128 x 128 FP64: 62 of the E
+// update's 69 us at the copy rate); launches and their gaps on small ones,
+// where the separate ghost fill cost 3.8 us per call, 15 us of a step.
 
-template <typename real>
-__global__ void __launch_bounds__(256) update_e_kernel(Geom g, real *__restrict__ ex, real *__restrict__ ey,
-                                                       real *__restrict__ ez, const real *__restrict__ bx,
-                                                       const real *__restrict__ by, const real *__restrict__ bz,
-                                                       const real *__restrict__ jx, const real *__restrict__ jy,
-                                                       const real *__restrict__ jz, real h, real idx, real idy,
-                                                       real idz) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    int k = blockIdx.z;
-    if (i >= g.n[0] || j >= g.n[1]) return;
-    i += g.mem;
-    j += g.mem;
-    k += g.mem;
-    const int c = g.fi(k, j, i), rc = g.ri(k, j, i);
-    const int sy = g.f[0], sz = g.fxy;
-    real bxc = bx[c], byc = by[c], bzc = bz[c];
-    ex[c] += h * ((bzc - bz[c - sy]) * idy - (byc - by[c - sz]) * idz - jx[rc]);
-    ey[c] += h * ((bxc - bx[c - sz]) * idz - (bzc - bz[c - 1]) * idx - jy[rc]);
-    ez[c] += h * ((byc - by[c - 1]) * idx - (bxc - bx[c - sy]) * idy - jz[rc]);
+// The points the threads of an update stand for: the physical cells, and
+// along non-periodic axes of a grid with periodic ones the ghosts too, whose
+// values (set by the boundary conditions) have periodic images.
+struct YeePoints {
+    int lo[3], ext[3];
+    int bx, by;            // blocks of 32 x 8 points along x and y
+    unsigned blocks;
+};
+
+static YeePoints yee_points(const Geom &g) {
+    YeePoints q{};
+    const bool any = g.per[0] || g.per[1] || g.per[2];
+    for (int d = 0; d < 3; ++d) {
+        const bool ghosts = any && !g.per[d];
+        q.lo[d] = ghosts ? 0 : g.mem;
+        q.ext[d] = ghosts ? g.f[d] : g.n[d];
+    }
+    q.bx = (q.ext[0] + 31) / 32;
+    q.by = (q.ext[1] + 7) / 8;
+    q.blocks = (unsigned)q.bx * (unsigned)q.by * (unsigned)q.ext[2];
+    return q;
 }
 
+// the point of this thread (blocks of 32 x 8 threads); false: none
+__device__ __forceinline__ bool yee_point(const YeePoints &q, unsigned block, int &i, int &j, int &k, const Geom &g,
+                                          bool &physical) {
+    const unsigned t = block / q.bx;
+    i = (int)(block - t * q.bx) * 32 + threadIdx.x;
+    k = (int)(t / q.by);
+    j = (int)(t - k * q.by) * 8 + threadIdx.y;
+    if (i >= q.ext[0] || j >= q.ext[1]) return false;
+    i += q.lo[0];
+    j += q.lo[1];
+    k += q.lo[2];
+    physical = i >= g.mem && i < g.n[0] + g.mem && j >= g.mem && j < g.n[1] + g.mem && k >= g.mem && k < g.n[2] + g.mem;
+    return true;
+}
+
+// Element offset to the one ghost image of physical coordinate c along a
+// periodic axis (0: none; n >= 2 mem + 2 leaves at most one).
+__device__ __forceinline__ int image_offset(const Geom &g, int d, int c, int stride) {
+    if (!g.per[d]) return 0;
+    return c < 2 * g.mem ? g.n[d] * stride : (c >= g.n[d] ? -g.n[d] * stride : 0);
+}
+
+// three values at element c and at all its periodic images (c itself only if
+// `self`)
 template <typename real>
-__global__ void __launch_bounds__(256) update_b_kernel(Geom g, const real *__restrict__ ex,
-                                                       const real *__restrict__ ey, const real *__restrict__ ez,
-                                                       real *__restrict__ bx, real *__restrict__ by,
-                                                       real *__restrict__ bz, real h, real idx, real idy, real idz) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int j = blockIdx.y * blockDim.y + threadIdx.y;
-    int k = blockIdx.z;
-    if (i >= g.n[0] || j >= g.n[1]) return;
-    i += g.mem;
-    j += g.mem;
-    k += g.mem;
+__device__ __forceinline__ void store_images(const Geom &g, int k, int j, int i, int c, bool self, real *a0, real *a1,
+                                             real *a2, real v0, real v1, real v2) {
+    const int ox = image_offset(g, 0, i, 1), oy = image_offset(g, 1, j, g.f[0]), oz = image_offset(g, 2, k, g.fxy);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        if (((b & 1) && !ox) || ((b & 2) && !oy) || ((b & 4) && !oz) || (b == 0 && !self)) continue;
+        const int at = c + (b & 1 ? ox : 0) + (b & 2 ? oy : 0) + (b & 4 ? oz : 0);
+        a0[at] = v0;
+        a1[at] = v1;
+        a2[at] = v2;
+    }
+}
+
+// twice: the last half of a step and the first half of the next in one pass
+// (the same B and J, two rounded additions)
+template <typename real>
+__global__ void __launch_bounds__(256) update_e_kernel(Geom g, YeePoints q, real *ex, real *ey, real *ez,
+                                                       const real *__restrict__ bx, const real *__restrict__ by,
+                                                       const real *__restrict__ bz, const real *__restrict__ jx,
+                                                       const real *__restrict__ jy, const real *__restrict__ jz,
+                                                       real h, real idx, real idy, real idz, int twice) {
+    int i, j, k;
+    bool physical;
+    if (!yee_point(q, blockIdx.x, i, j, k, g, physical)) return;
     const int c = g.fi(k, j, i);
-    const int sy = g.f[0], sz = g.fxy;
-    real exc = ex[c], eyc = ey[c], ezc = ez[c];
-    bx[c] -= h * ((ez[c + sy] - ezc) * idy - (ey[c + sz] - eyc) * idz);
-    by[c] -= h * ((ex[c + sz] - exc) * idz - (ez[c + 1] - ezc) * idx);
-    bz[c] -= h * ((ey[c + 1] - eyc) * idx - (ex[c + sy] - exc) * idy);
+    real vx = ex[c], vy = ey[c], vz = ez[c];
+    if (physical) {
+        const int rc = g.ri(k, j, i), sy = g.f[0], sz = g.fxy;
+        const real bxc = bx[c], byc = by[c], bzc = bz[c];
+        const real rx = (bzc - bz[c - sy]) * idy - (byc - by[c - sz]) * idz - jx[rc];
+        const real ry = (bxc - bx[c - sz]) * idz - (bzc - bz[c - 1]) * idx - jy[rc];
+        const real rz = (byc - by[c - 1]) * idx - (bxc - bx[c - sy]) * idy - jz[rc];
+        vx += h * rx;
+        vy += h * ry;
+        vz += h * rz;
+        if (twice) {
+            vx += h * rx;
+            vy += h * ry;
+            vz += h * rz;
+        }
+    }
+    store_images(g, k, j, i, c, physical, ex, ey, ez, vx, vy, vz);
 }
 
 // ---------------------------------------------------------------------------
-// Periodic ghost fill (single-rank meaning of exchange_boundary_data,
-// src/mpi_utils.cpp:9-60).  The reference copies X, then Y, then Z slabs over
+// Periodic ghost fill of one array on its own (single-rank meaning of
+// exchange_boundary_data, src/mpi_utils.cpp:9-60).  The reference copies X, then Y, then Z slabs over
 // the full extent of the other dimensions; the result is that every point
 // whose coordinate in a periodic dimension is a ghost holds the value of the
 // point with each such coordinate replaced by its periodic image (other
@@ -199,40 +258,98 @@ static ShellPlan fold_plan(const Geom &g) {
     return pl;
 }
 
+// element offset to the one image of ring coordinate c along a periodic axis
+// (0: none)
+__device__ __forceinline__ int fold_offset(const Geom &g, int d, int c, int stride) {
+    if (!g.per[d]) return 0;
+    return c >= g.n[d] - 1 ? -g.n[d] * stride : (c <= 2 * g.mem ? g.n[d] * stride : 0);
+}
+
+// the current arrays an auxiliary part of a launch works on
 template <typename real>
-__global__ void fold_kernel(Geom g, ShellPlan pl, real *a0, real *a1, real *a2, real *a3, real *a4) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= pl.start[pl.ns]) return;
-    real *arr[5] = {a0, a1, a2, a3, a4};
-    real *a = arr[blockIdx.y];
-    if (!a) return;
+struct RingWork {
+    ShellPlan pl;            // fold
+    real *a[5];
+    int na;
+    long long words;         // clear: 16-byte words of one array
+};
+
+// owner point t of the fold plan, every array: all loads of a point are
+// issued before its stores
+template <typename real>
+__device__ __forceinline__ void fold_point(const Geom &g, const RingWork<real> &w, unsigned t) {
+    const ShellPlan &pl = w.pl;
     int s = 0;
-    while (s + 1 < pl.ns && t >= pl.start[s + 1]) ++s;
-    long long l = t - pl.start[s];
+    while (s + 1 < pl.ns && (long long)t >= pl.start[s + 1]) ++s;
+    unsigned l = t - (unsigned)pl.start[s];
     int c[3];
+#pragma unroll
     for (int e = 0; e < 3; ++e) {
-        int q = (int)(l % pl.ext[s][e]);
-        l /= pl.ext[s][e];
-        c[e] = pl.lo[s][e] + q;
+        const unsigned x = (unsigned)pl.ext[s][e], r = l / x;
+        c[e] = pl.lo[s][e] + (int)(l - r * x);
+        l = r;
+        if (e == pl.dim[s]) c[e] = c[e] <= g.mem ? g.mem + c[e] : g.n[e] - 1 + (c[e] - g.mem - 1);
     }
-    const int d = pl.dim[s];
-    c[d] = c[d] <= g.mem ? g.mem + c[d] : g.n[d] - 1 + (c[d] - g.mem - 1);
-    int img[3][2], nimg[3];
-    for (int e = 0; e < 3; ++e) {
-        img[e][0] = c[e];
-        nimg[e] = 1;
-        if (g.per[e]) {
-            if (c[e] >= g.n[e] - 1) img[e][nimg[e]++] = c[e] - g.n[e];
-            else if (c[e] <= 2 * g.mem) img[e][nimg[e]++] = c[e] + g.n[e];
+    const int at = g.ri(c[2], c[1], c[0]);
+    const int ox = fold_offset(g, 0, c[0], 1), oy = fold_offset(g, 1, c[1], g.r[0]), oz = fold_offset(g, 2, c[2], g.rxy);
+    for (int q = 0; q < w.na; ++q) {
+        real *a = w.a[q] + at, v[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            const bool on = !((b & 1) && !ox) && !((b & 2) && !oy) && !((b & 4) && !oz);
+            v[b] = on ? a[(b & 1 ? ox : 0) + (b & 2 ? oy : 0) + (b & 4 ? oz : 0)] : real(0);
         }
+        real tot = v[0];
+#pragma unroll
+        for (int b = 1; b < 8; ++b) tot += v[b];
+#pragma unroll
+        for (int b = 0; b < 8; ++b)
+            if (!((b & 1) && !ox) && !((b & 2) && !oy) && !((b & 4) && !oz))
+                a[(b & 1 ? ox : 0) + (b & 2 ? oy : 0) + (b & 4 ? oz : 0)] = tot;
     }
-    real tot = 0;
-    for (int z = 0; z < nimg[2]; ++z)
-        for (int y = 0; y < nimg[1]; ++y)
-            for (int x = 0; x < nimg[0]; ++x) tot += a[g.ri(img[2][z], img[1][y], img[0][x])];
-    for (int z = 0; z < nimg[2]; ++z)
-        for (int y = 0; y < nimg[1]; ++y)
-            for (int x = 0; x < nimg[0]; ++x) a[g.ri(img[2][z], img[1][y], img[0][x])] = tot;
+}
+
+template <typename real>
+__global__ void __launch_bounds__(256) fold_kernel(Geom g, const __grid_constant__ RingWork<real> w) {
+    const unsigned t = blockIdx.x * 256u + threadIdx.x;
+    if ((long long)t < w.pl.start[w.pl.ns]) fold_point(g, w, t);
+}
+
+// B update (and its periodic images).  The blocks beyond it work on the
+// current arrays, which B neither reads nor writes: after the E update has
+// used them they are cleared (the first half of a step), or the push's
+// deposits are folded (the second half).  Launched alone, the three clears
+// and the fold cost 4 and 8 us of a 32^3 step.
+enum : int { kBesideNone = 0, kBesideClear = 1, kBesideFold = 2 };
+template <typename real, int BESIDE>
+__global__ void __launch_bounds__(256) update_b_kernel(Geom g, YeePoints q, const real *__restrict__ ex,
+                                                       const real *__restrict__ ey, const real *__restrict__ ez,
+                                                       real *bx, real *by, real *bz, real h, real idx, real idy,
+                                                       real idz, const __grid_constant__ RingWork<real> w) {
+    if (BESIDE != kBesideNone && blockIdx.x >= q.blocks) {
+        const unsigned t = (blockIdx.x - q.blocks) * 256u + threadIdx.y * 32u + threadIdx.x;
+        if constexpr (BESIDE == kBesideFold) {
+            if ((long long)t < w.pl.start[w.pl.ns]) fold_point(g, w, t);
+        } else {
+            const unsigned nt = (gridDim.x - q.blocks) * 256u;
+            for (int a = 0; a < w.na; ++a)
+                for (long long e = t; e < w.words; e += nt) reinterpret_cast<uint4 *>(w.a[a])[e] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        return;
+    }
+    int i, j, k;
+    bool physical;
+    if (!yee_point(q, blockIdx.x, i, j, k, g, physical)) return;
+    const int c = g.fi(k, j, i);
+    real vx = bx[c], vy = by[c], vz = bz[c];
+    if (physical) {
+        const int sy = g.f[0], sz = g.fxy;
+        const real exc = ex[c], eyc = ey[c], ezc = ez[c];
+        vx -= h * ((ez[c + sy] - ezc) * idy - (ey[c + sz] - eyc) * idz);
+        vy -= h * ((ex[c + sz] - exc) * idz - (ez[c + 1] - ezc) * idx);
+        vz -= h * ((ey[c + 1] - eyc) * idx - (ex[c + sy] - exc) * idy);
+    }
+    store_images(g, k, j, i, c, physical, bx, by, bz, vx, vy, vz);
 }
 
 // ---------------------------------------------------------------------------
@@ -435,24 +552,41 @@ void launch_absorbing_faces(pic_ctx *c) {
 // host launchers
 
 template <typename real>
-static void fields_e(pic_ctx *c, double coef) {
-    const Geom &g = c->g;
-    dim3 blk(32, 8), grd((g.n[0] + 31) / 32, (g.n[1] + 7) / 8, g.n[2]);
+static void fields_e(pic_ctx *c, double coef, bool twice) {
+    const YeePoints q = yee_points(c->g);
     real **F = (real **)c->field;
     real **R = (real **)c->ring;
-    update_e_kernel<real><<<grd, blk, 0, c->stream>>>(g, F[0], F[1], F[2], F[3], F[4], F[5], R[0], R[1], R[2],
-                                                      (real)coef, (real)(1.0 / c->p.dx),
-                                                      (real)(1.0 / c->p.dy), (real)(1.0 / c->p.dz));
+    update_e_kernel<real><<<q.blocks, dim3(32, 8), 0, c->stream>>>(
+        c->g, q, F[0], F[1], F[2], F[3], F[4], F[5], R[0], R[1], R[2], (real)coef, (real)(1.0 / c->p.dx),
+        (real)(1.0 / c->p.dy), (real)(1.0 / c->p.dz), twice ? 1 : 0);
+}
+
+// the selected ring arrays (bit k of mask: jx, jy, jz, rho0, rho1)
+template <typename real>
+static RingWork<real> ring_work(const pic_ctx *c, unsigned mask) {
+    RingWork<real> w{};
+    w.pl = fold_plan(c->g);
+    for (int k = 0; k < 5; ++k)
+        if (mask >> k & 1u) w.a[w.na++] = (real *)c->ring[k];
+    w.words = (c->g.rsz * (long long)sizeof(real) + 15) / 16;   // (allocations are rounded up)
+    return w;
 }
 
 template <typename real>
-static void fields_b(pic_ctx *c, double coef) {
-    const Geom &g = c->g;
-    dim3 blk(32, 8), grd((g.n[0] + 31) / 32, (g.n[1] + 7) / 8, g.n[2]);
+static void fields_b(pic_ctx *c, double coef, int beside, unsigned mask) {
+    const YeePoints q = yee_points(c->g);
     real **F = (real **)c->field;
-    update_b_kernel<real><<<grd, blk, 0, c->stream>>>(g, F[0], F[1], F[2], F[3], F[4], F[5], (real)coef,
-                                                      (real)(1.0 / c->p.dx), (real)(1.0 / c->p.dy),
-                                                      (real)(1.0 / c->p.dz));
+    const RingWork<real> w = ring_work<real>(c, mask);
+    const long long nf = w.pl.start[w.pl.ns];
+    auto launch = [&](auto kernel, long long extra) {
+        kernel<<<q.blocks + (unsigned)extra, dim3(32, 8), 0, c->stream>>>(
+            c->g, q, F[0], F[1], F[2], F[3], F[4], F[5], (real)coef, (real)(1.0 / c->p.dx), (real)(1.0 / c->p.dy),
+            (real)(1.0 / c->p.dz), w);
+    };
+    // clearing: about four 16-byte stores per thread and array, at most 4 blocks per SM
+    if (beside == kBesideClear) launch(update_b_kernel<real, kBesideClear>, std::min((w.words + 1023) / 1024, 148ll * 4));
+    else if (beside == kBesideFold && nf) launch(update_b_kernel<real, kBesideFold>, (nf + 255) / 256);
+    else launch(update_b_kernel<real, kBesideNone>, 0);
 }
 
 // ghost fill of up to three field arrays (null entries skipped)
@@ -469,23 +603,21 @@ static void ghost_fill_any(pic_ctx *c, void *a0, void *a1, void *a2) {
     if (c->fp32) ghost_fill<float>(c, a0, a1, a2); else ghost_fill<double>(c, a0, a1, a2);
 }
 
-void launch_update_e(pic_ctx *c, double coef) {
+void launch_update_e(pic_ctx *c, double coef, bool twice) {
     prof_begin(c, "yee_update_e");
-    if (c->fp32) fields_e<float>(c, coef); else fields_e<double>(c, coef);
-    prof_end(c);
-    prof_begin(c, "ghost_fill");
-    ghost_fill_any(c, c->field[0], c->field[1], c->field[2]);
+    if (c->fp32) fields_e<float>(c, coef, twice); else fields_e<double>(c, coef, twice);
     prof_end(c);
 }
 
-void launch_update_b(pic_ctx *c, double coef) {
+static void update_b_with(pic_ctx *c, double coef, int beside, unsigned mask) {
     prof_begin(c, "yee_update_b");
-    if (c->fp32) fields_b<float>(c, coef); else fields_b<double>(c, coef);
-    prof_end(c);
-    prof_begin(c, "ghost_fill");
-    ghost_fill_any(c, c->field[3], c->field[4], c->field[5]);
+    if (c->fp32) fields_b<float>(c, coef, beside, mask); else fields_b<double>(c, coef, beside, mask);
     prof_end(c);
 }
+
+void launch_update_b(pic_ctx *c, double coef) { update_b_with(c, coef, kBesideNone, 0); }
+void launch_update_b_clear(pic_ctx *c, double coef, unsigned mask) { update_b_with(c, coef, kBesideClear, mask); }
+void launch_update_b_fold(pic_ctx *c, double coef, unsigned mask) { update_b_with(c, coef, kBesideFold, mask); }
 
 void launch_ghost_fill_one(pic_ctx *c, int array) {
     prof_begin(c, "ghost_fill");
@@ -493,16 +625,12 @@ void launch_ghost_fill_one(pic_ctx *c, int array) {
     prof_end(c);
 }
 
-// fold of the ring arrays selected by `mask` (bit k: jx, jy, jz, rho0, rho1)
+// fold of the ring arrays selected by `mask`
 template <typename real>
 static void fold(pic_ctx *c, unsigned mask) {
-    ShellPlan pl = fold_plan(c->g);
-    long long n = pl.start[pl.ns];
-    if (n == 0) return;
-    real *R[5];
-    for (int k = 0; k < 5; ++k) R[k] = (mask >> k & 1u) ? (real *)c->ring[k] : nullptr;
-    dim3 grd((unsigned)((n + 255) / 256), 5);
-    fold_kernel<real><<<grd, 256, 0, c->stream>>>(c->g, pl, R[0], R[1], R[2], R[3], R[4]);
+    const RingWork<real> w = ring_work<real>(c, mask);
+    const long long n = w.pl.start[w.pl.ns];
+    if (n) fold_kernel<real><<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->g, w);
 }
 
 void launch_fold_currents(pic_ctx *c, unsigned mask) {

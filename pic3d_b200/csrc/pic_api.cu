@@ -558,7 +558,7 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     const size_t rs = real_size(c);
     int r = PIC_OK;
     for (int k = 0; k < 6 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->field[k], (size_t)c->g.fsz * rs);
-    for (int k = 0; k < 5 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->ring[k], (size_t)c->g.rsz * rs);
+    for (int k = 0; k < 5 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->ring[k], ((size_t)c->g.rsz * rs + 15) / 16 * 16);
     r = r ? r : dalloc(c, &c->d_status, sizeof(unsigned));
     r = r ? r : dalloc(c, &c->d_scratch_ll, 8 * sizeof(long long));
     r = r ? r : dalloc(c, &c->d_diag, PIC_NDIAG * sizeof(double));
@@ -1046,27 +1046,36 @@ int pic_initial_push(pic_ctx *c) {
 // One iteration of run_main_time_loop.  rho (a diagnostic: it never feeds
 // the fields) is cleared, deposited and folded only when the step's rho can
 // be observed, i.e. on the last step of a pic_run_steps call.
-static int run_one_step(pic_ctx *c, bool rho_observed) {
+// e_first: the first E half-update is still to do.  e_next: a step follows
+// whose first E half-update directly follows this step's second one (nothing
+// between them writes a field): both are then done here in one pass.
+static int run_one_step(pic_ctx *c, bool rho_observed, bool e_first, bool e_next) {
     c->step += 1;
     c->rho_skip = !rho_observed && !c->p.adjoint;
+    const unsigned rings = c->rho_skip ? 7u : 31u;
     int r;
     if ((r = pic_radiating_boundary(c, 1, 0, c->step))) return r;
-    if ((r = pic_update_fields_first(c))) return r;
-    if ((r = pic_clear_currents(c))) return r;
+    if (e_first) launch_update_e(c, c->p.dt_half);
+    launch_update_b_clear(c, c->p.dt_half, rings);
+    if ((r = launch_check(c, "update_fields_first"))) return r;
     launch_sort_due(c, 3);
     adjoint_record_hook(c);
     if ((r = push_both(c))) return r;
     if ((r = pic_exchange_particles(c, 0))) return r;
     if ((r = pic_exchange_particles(c, 1))) return r;
-    if ((r = pic_exchange_currents(c))) return r;
-    return pic_update_fields_second(c);
+    launch_update_b_fold(c, c->p.dt_half, rings);
+    launch_update_e(c, c->p.dt_half, e_next);
+    return launch_check(c, "update_fields_second");
 }
 
 int pic_run_steps(pic_ctx *c, int nsteps) {
     if (!c || nsteps < 0) return PIC_EINVAL;
     cudaSetDevice(c->device);
+    // with every face periodic no boundary condition comes between two steps;
+    // adjoint contexts record the fields of each step as they are
+    const bool merge = c->g.per[0] && c->g.per[1] && c->g.per[2] && !c->p.adjoint;
     for (int t = 0; t < nsteps; ++t) {
-        int r = run_one_step(c, t + 1 == nsteps);
+        int r = run_one_step(c, t + 1 == nsteps, !merge || t == 0, merge && t + 1 < nsteps);
         c->rho_skip = false;
         if (r) return r;
     }

@@ -10,8 +10,11 @@ void prof_begin(pic_ctx *c, const char *name);
 void prof_end(pic_ctx *c);
 
 // field_kernels.cu
-void launch_update_e(pic_ctx *c, double coef);   // E += coef (curl B - J), then the E ghost fill
-void launch_update_b(pic_ctx *c, double coef);   // B -= coef curl E, then the B ghost fill
+void launch_update_e(pic_ctx *c, double coef, bool twice = false);   // E += coef (curl B - J), with its ghosts
+void launch_update_b(pic_ctx *c, double coef);   // B -= coef curl E, with its ghosts
+// the same beside work on the ring arrays of `mask` (bits: jx, jy, jz, rho0, rho1)
+void launch_update_b_clear(pic_ctx *c, double coef, unsigned mask);
+void launch_update_b_fold(pic_ctx *c, double coef, unsigned mask);
 void launch_ghost_fill_one(pic_ctx *c, int array);
 void launch_fold_currents(pic_ctx *c, unsigned mask = 31u);
 void launch_radiating_boundary(pic_ctx *c, int is_left, int is_right, int step);
