@@ -7,13 +7,15 @@
 // components through the read-only path; the deposit adds J (and rho) with
 // hardware atomics into the ring buffers, which the fold kernel then
 // completes for periodic faces exactly as the reference's ghost exchange.
+#include <algorithm>
+
 #include "pic_kernels.cuh"
 #include "push_core.cuh"
 
 namespace pic {
 
 template <typename real, int P, bool SPIN>
-__global__ void __launch_bounds__(256) push_kernel(PushArgs<real> a) {
+__device__ __forceinline__ void push_all(const PushArgs<real> &a) {
     constexpr int H = P / 2;
     const long long n = *a.count;
     View<const real> fv[6];
@@ -38,6 +40,17 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs<real> a) {
     }
 }
 
+// the arguments of up to two species (blockIdx.y)
+template <typename real>
+struct PushPair {
+    PushArgs<real> s[2];
+};
+
+template <typename real, int P, bool SPIN>
+__global__ void __launch_bounds__(256) push_kernel(const __grid_constant__ PushPair<real> a) {
+    push_all<real, P, SPIN>(a.s[blockIdx.y]);
+}
+
 // ---------------------------------------------------------------------------
 
 static int sm_count(pic_ctx *c) {
@@ -49,7 +62,8 @@ static int sm_count(pic_ctx *c) {
 template <typename real, int P, bool SPIN>
 static void push_t(pic_ctx *c, int kind) {
     Species &s = c->sp[kind];
-    PushArgs<real> a = make_push_args<real>(c, kind);
+    PushPair<real> a{};
+    a.s[0] = make_push_args<real>(c, kind);
     long long n = s.n_host;
     if (n > 0) {
         long long blocks = (n + 255) / 256;
@@ -59,33 +73,38 @@ static void push_t(pic_ctx *c, int kind) {
     s.cur = 1 - s.cur;
 }
 
-// the particles listed in idx as (index, home tile) pairs (count on the
-// device): those the tiled kernel left to the global kernel; each one that
-// ends away from its home tile is recorded as a visitor (when vsink is on)
+// The particles that the tile kernel left to the global kernel, (index, home
+// tile) pairs counted on the device; each one that ends away from its home
+// tile is recorded as a visitor (when the species has visitor lists).
 template <typename real, int P, bool SPIN>
-static void push_list_t(pic_ctx *c, int kind, const int *idx, const unsigned long long *count, const VisSink &vsink) {
-    Species &s = c->sp[kind];
-    PushArgs<real> a = make_push_args<real>(c, kind);
-    a.idx = idx;
-    a.idx_pairs = 1;
-    a.vsink = vsink;
-    a.count = reinterpret_cast<const long long *>(count);
-    long long n = s.n_host;
-    if (n > 0) {
-        long long blocks = (n + 255) / 256;
-        long long maxb = (long long)sm_count(c) * 4;
-        push_kernel<real, P, SPIN><<<(unsigned)(blocks < maxb ? blocks : maxb), 256, 0, c->stream>>>(a);
+static void push_stragglers_t(pic_ctx *c, int mask) {
+    PushPair<real> a{};
+    unsigned ns = 0;
+    long long n = 0;
+    for (int k = 0; k < 2; ++k) {
+        Species &s = c->sp[k];
+        if (!((mask >> k) & 1) || s.n_host <= 0) continue;
+        PushArgs<real> &q = a.s[ns++];
+        q = make_push_args<real>(c, k);
+        q.idx = s.strag;
+        q.idx_pairs = 1;
+        q.vsink = vis_sink_of(c, s);
+        q.count = reinterpret_cast<const long long *>(c->d_nstrag + k);
+        n = std::max<long long>(n, s.n_host);
     }
+    if (!ns) return;
+    const long long blocks = (n + 255) / 256, maxb = (long long)sm_count(c) * 4;
+    push_kernel<real, P, SPIN><<<dim3((unsigned)std::min(blocks, maxb), ns), 256, 0, c->stream>>>(a);
 }
 
-void launch_push_list(pic_ctx *c, int kind, const int *idx, const unsigned long long *count, const VisSink &v) {
-    bool spin = spin_active(c, kind);
+void launch_push_stragglers(pic_ctx *c, int mask) {
+    const bool spin = ((mask & 1) && spin_active(c, 0)) || ((mask & 2) && spin_active(c, 1));
     if (c->fp32) {
-        if (c->order == 2) spin ? push_list_t<float, 3, true>(c, kind, idx, count, v) : push_list_t<float, 3, false>(c, kind, idx, count, v);
-        else spin ? push_list_t<float, 5, true>(c, kind, idx, count, v) : push_list_t<float, 5, false>(c, kind, idx, count, v);
+        if (c->order == 2) spin ? push_stragglers_t<float, 3, true>(c, mask) : push_stragglers_t<float, 3, false>(c, mask);
+        else spin ? push_stragglers_t<float, 5, true>(c, mask) : push_stragglers_t<float, 5, false>(c, mask);
     } else {
-        if (c->order == 2) spin ? push_list_t<double, 3, true>(c, kind, idx, count, v) : push_list_t<double, 3, false>(c, kind, idx, count, v);
-        else spin ? push_list_t<double, 5, true>(c, kind, idx, count, v) : push_list_t<double, 5, false>(c, kind, idx, count, v);
+        if (c->order == 2) spin ? push_stragglers_t<double, 3, true>(c, mask) : push_stragglers_t<double, 3, false>(c, mask);
+        else spin ? push_stragglers_t<double, 5, true>(c, mask) : push_stragglers_t<double, 5, false>(c, mask);
     }
 }
 
@@ -107,81 +126,106 @@ void launch_push(pic_ctx *c, int kind) {
 // exchange_particle_data, src/mpi_utils.cpp:62-230, on one rank): a particle
 // with x < 0 or x >= n along a non-periodic axis is dropped.  Holes below the
 // new count are filled from survivors above it (order is not preserved).
+//
+// One pass over the positions lists the particles to drop; what follows is
+// work on that list and on as many particles at the end of the arrays.  Each
+// launch serves up to two species (blockIdx.y).  (A second pass over all
+// positions and one thread moving a particle's thirteen values one after the
+// other cost 2 x 20 us of a 45 x 38 x 51 step.)
 
 struct RemoveArgs {
     Geom g;
     CellPack cp;
     int fp32;
-    long long *count;         // in/out
-    long long *ctr;           // [0] removed, [1] holes, [2] movers
-    int *holes, *movers;
-    const double *x, *y, *z;
-    const int *cell;
-    const float *ox, *oy, *oz;
+    struct One {
+        long long *count;         // in/out
+        long long *ctr;           // [0] dropped, [1] holes, [2] movers
+        // One buffer of 2 cap indices: nd dropped from the front, the holes
+        // after them, the movers backwards from the end.  Holes and movers
+        // are at most min(nd, n - nd) each: 3/2 n indices in all.
+        int *list;
+        long long cap;
+        const double *x, *y, *z;
+        const int *cell;
+        const float *ox, *oy, *oz;
+        unsigned char *dead;      // adjoint mode: flags instead of lists
+        // the moved particles' arrays
+        void *a[16];
+        int bytes[16], na;
+        // visitor lists (vsink.raw null: none): a moved particle now belongs to
+        // the sorted slice of the tile whose range holds its hole
+        VisSink vsink;
+        const unsigned *offs;     // per-key start offsets of the last sort
+        long long keys_per_tile;
+    } s[2];
 };
 
-__device__ __forceinline__ bool is_dead(const RemoveArgs &a, long long i) {
-    if (a.fp32) {
-        int cx, cy, cz;
-        a.cp.unpack(a.cell[i], cx, cy, cz);
-        int c[3] = {cx, cy, cz};
+__device__ __forceinline__ bool is_dead(const RemoveArgs &r, const RemoveArgs::One &a, long long i) {
+    if (r.fp32) {
+        int c[3];
+        r.cp.unpack(a.cell[i], c[0], c[1], c[2]);
         bool dead = false;
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-            if (!a.g.per[d]) dead = dead || c[d] < 0 || c[d] >= a.g.n[d];
+            if (!r.g.per[d]) dead = dead || c[d] < 0 || c[d] >= r.g.n[d];
         return dead;
     }
-    double c[3] = {a.x[i], a.y[i], a.z[i]};
+    const double *x[3] = {a.x, a.y, a.z};
     bool dead = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-        if (!a.g.per[d]) dead = dead || c[d] < 0.0 || c[d] >= (double)a.g.n[d];
+        if (!r.g.per[d]) {
+            const double v = x[d][i];
+            dead = dead || v < 0.0 || v >= (double)r.g.n[d];
+        }
     return dead;
 }
 
-__global__ void count_dead_kernel(RemoveArgs a) {
-    long long n = *a.count;
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool dead = i < n && is_dead(a, i);
-    unsigned m = __ballot_sync(0xffffffffu, dead);
-    if ((threadIdx.x & 31) == 0 && m) atomicAdd((unsigned long long *)&a.ctr[0], (unsigned long long)__popc(m));
+__global__ void __launch_bounds__(256) list_dead_kernel(const __grid_constant__ RemoveArgs r) {
+    const RemoveArgs::One &a = r.s[blockIdx.y];
+    const long long n = *a.count;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool dead = i < n && is_dead(r, a, i);
+    const unsigned m = __ballot_sync(0xffffffffu, dead);
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd((unsigned long long *)&a.ctr[0], (unsigned long long)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (dead) a.list[base + __popc(m & ((1u << lane) - 1u))] = (int)i;
 }
 
-__global__ void list_moves_kernel(RemoveArgs a) {
-    long long n = *a.count;
-    long long nn = n - a.ctr[0];
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    bool dead = is_dead(a, i);
-    if (i < nn && dead) a.holes[atomicAdd((unsigned long long *)&a.ctr[1], 1ull)] = (int)i;
-    if (i >= nn && !dead) a.movers[atomicAdd((unsigned long long *)&a.ctr[2], 1ull)] = (int)i;
+// Holes, movers, and the visitor entries of particles that the compaction
+// removes or moves, which are dropped (tile -1); apply_moves records the
+// moved ones anew.
+__global__ void __launch_bounds__(256) list_moves_kernel(const __grid_constant__ RemoveArgs r) {
+    const RemoveArgs::One &a = r.s[blockIdx.y];
+    const long long n = *a.count, nd = a.ctr[0], nn = n - nd;
+    if (nd == 0) return;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    for (long long e = t0; e < nd; e += nt) {
+        const int i = a.list[e];
+        if (i < nn) a.list[nd + (long long)atomicAdd((unsigned long long *)&a.ctr[1], 1ull)] = i;
+        if (!is_dead(r, a, nn + e))
+            a.list[2 * a.cap - 1 - (long long)atomicAdd((unsigned long long *)&a.ctr[2], 1ull)] = (int)(nn + e);
+    }
+    if (!a.vsink.raw) return;
+    const long long ne = min((long long)*a.vsink.nraw, a.vsink.cap);
+    for (long long e = t0; e < ne; e += nt) {
+        const long long i = a.vsink.raw[3 * e];
+        if (i >= nn || is_dead(r, a, i)) {
+            atomicSub(a.vsink.cnt + a.vsink.raw[3 * e + 2], 1u);
+            a.vsink.raw[3 * e + 2] = -1;
+        }
+    }
 }
-
-template <typename T>
-__device__ __forceinline__ void mv(T *p, int dst, int src) {
-    if (p) p[dst] = p[src];
-}
-
-struct MoveArgs {
-    long long *ctr;
-    long long *count;
-    const int *holes, *movers;
-    double *d[16];
-    float *f[16];
-    int *i[3];
-    // visitor lists (vsink.raw null: none): a moved particle now belongs to
-    // the sorted slice of the tile whose range holds its hole
-    VisSink vsink;
-    RemoveArgs at;          // the moved particle's position (current buffer)
-    const unsigned *offs;   // per-key start offsets of the last sort
-    long long keys_per_tile;
-};
 
 // the cell and the node the next push's decode will see (as push_move
 // reports them)
-__device__ __forceinline__ void current_cell(const RemoveArgs &a, long long i, int (&c)[3], int (&nd)[3]) {
-    if (a.fp32) {
-        a.cp.unpack(a.cell[i], c[0], c[1], c[2]);
+__device__ __forceinline__ void current_cell(const RemoveArgs &r, const RemoveArgs::One &a, long long i, int (&c)[3],
+                                             int (&nd)[3]) {
+    if (r.fp32) {
+        r.cp.unpack(a.cell[i], c[0], c[1], c[2]);
         const float o[3] = {a.ox[i], a.oy[i], a.oz[i]};
 #pragma unroll
         for (int d = 0; d < 3; ++d) nd[d] = c[d] + (o[d] >= 0.5f ? 1 : 0);
@@ -191,13 +235,13 @@ __device__ __forceinline__ void current_cell(const RemoveArgs &a, long long i, i
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         double v = v0[d];
-        if (a.g.per[d]) {
-            if (v < 0.0) v += a.g.n[d];
-            if (v > (double)a.g.n[d]) v -= a.g.n[d];
+        if (r.g.per[d]) {
+            if (v < 0.0) v += r.g.n[d];
+            if (v > (double)r.g.n[d]) v -= r.g.n[d];
         }
-        const double xc = v - (double)(1 - a.g.mem);
-        c[d] = xc >= 0.0 ? (int)xc - (a.g.mem - 1) : -1;
-        nd[d] = xc >= 0.0 ? (int)(xc + 0.5) - (a.g.mem - 1) : -1;
+        const double xc = v - (double)(1 - r.g.mem);
+        c[d] = xc >= 0.0 ? (int)xc - (r.g.mem - 1) : -1;
+        nd[d] = xc >= 0.0 ? (int)(xc + 0.5) - (r.g.mem - 1) : -1;
     }
 }
 
@@ -212,113 +256,93 @@ __device__ __forceinline__ int home_tile(const unsigned *offs, long long keys_pe
     return lo;
 }
 
-__global__ void apply_moves_kernel(MoveArgs a) {
-    long long m = a.ctr[2];
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    int dst = a.holes[t], src = a.movers[t];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        mv(a.d[k], dst, src);
-        mv(a.f[k], dst, src);
+// 16 lanes move a particle, one array each
+__global__ void __launch_bounds__(256) apply_moves_kernel(const __grid_constant__ RemoveArgs r) {
+    const RemoveArgs::One &a = r.s[blockIdx.y];
+    const long long nd = a.ctr[0], m = a.ctr[2];
+    const int k = threadIdx.x & 15;
+    for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4; t < m;
+         t += ((long long)gridDim.x * blockDim.x) >> 4) {
+        const int dst = a.list[nd + t], src = a.list[2 * a.cap - 1 - t];
+        if (k < a.na) {
+            if (a.bytes[k] == 8) ((double *)a.a[k])[dst] = ((const double *)a.a[k])[src];
+            else ((unsigned *)a.a[k])[dst] = ((const unsigned *)a.a[k])[src];
+        }
+        if (k == 15 && a.vsink.raw) {
+            int c[3], nd3[3];
+            current_cell(r, a, src, c, nd3);
+            const int nt = a.vsink.nt[0] * a.vsink.nt[1] * a.vsink.nt[2];
+            vis_note(a.vsink, r.g, dst, home_tile(a.offs, a.keys_per_tile, nt, dst), c, nd3);
+        }
     }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) mv(a.i[k], dst, src);
-    if (a.vsink.raw) {
-        int c[3], nd[3];
-        current_cell(a.at, src, c, nd);
-        const int nt = a.vsink.nt[0] * a.vsink.nt[1] * a.vsink.nt[2];
-        vis_note(a.vsink, a.at.g, dst, home_tile(a.offs, a.keys_per_tile, nt, dst), c, nd);
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.count -= nd;
 }
 
-// Entries the push recorded for particles that the compaction removes or
-// moves are dropped (tile -1); apply_moves records the moved ones anew.
-__global__ void vis_drop_kernel(RemoveArgs a, int *raw, const VisState *vs, long long cap) {
-    const long long n = *a.count, nn = n - a.ctr[0];
-    const long long ne = min((long long)vs->nraw, cap);
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (long long)gridDim.x * blockDim.x) {
-        const long long i = raw[3 * e];
-        if (i >= nn || is_dead(a, i)) raw[3 * e + 2] = -1;
-    }
+__global__ void __launch_bounds__(256) mark_dead_kernel(const __grid_constant__ RemoveArgs r) {
+    const RemoveArgs::One &a = r.s[blockIdx.y];
+    const long long n = *a.count;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && !a.dead[i] && is_dead(r, a, i)) a.dead[i] = 1;
 }
 
-__global__ void finish_remove_kernel(long long *count, long long *ctr) { *count = *count - ctr[0]; }
-
-__global__ void mark_dead_kernel(RemoveArgs a, unsigned char *dead) {
-    long long n = *a.count;
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && !dead[i] && is_dead(a, i)) dead[i] = 1;
-}
-
-void launch_remove(pic_ctx *c, int kind) {
+void launch_remove(pic_ctx *c, int mask) {
     const Geom &g = c->g;
     if (g.per[0] && g.per[1] && g.per[2]) return;
-    Species &s = c->sp[kind];
-    long long n = s.n_host;
-    if (n == 0) return;
-    if (s.dead) {
-        // adjoint mode: particle indices must stay stable across steps
-        RemoveArgs a{};
-        a.g = g;
-        a.cp = c->cp;
-        a.fp32 = c->fp32;
+    RemoveArgs r{};
+    r.g = g;
+    r.cp = c->cp;
+    r.fp32 = c->fp32;
+    unsigned ns = 0;
+    long long n = 0;
+    bool dead = false;
+    long long *ctr = c->d_scratch_ll + 8;
+    for (int kind = 0; kind < 2; ++kind) {
+        Species &s = c->sp[kind];
+        if (!((mask >> kind) & 1) || s.n_host == 0) continue;
+        RemoveArgs::One &a = r.s[ns];
         a.count = s.d_count;
-        a.x = s.a.x[s.cur]; a.y = s.a.y[s.cur]; a.z = s.a.z[s.cur];
-        a.cell = s.a.cell[s.cur];
+        a.ctr = ctr + 3 * ns++;
+        a.list = s.strag;
+        a.cap = s.cap;
+        const int cu = s.cur;
+        a.x = s.a.x[cu]; a.y = s.a.y[cu]; a.z = s.a.z[cu];
+        a.cell = s.a.cell[cu];
+        a.ox = s.a.ox[cu]; a.oy = s.a.oy[cu]; a.oz = s.a.oz[cu];
+        a.dead = s.dead;
+        dead = s.dead != nullptr;
+        auto add = [&](void *p, int bytes) {
+            if (!p) return;
+            a.a[a.na] = p;
+            a.bytes[a.na++] = bytes;
+        };
+        const int rs = c->fp32 ? 4 : 8;
+        for (int b = 0; b < 2; ++b) {
+            add(s.a.x[b], 8); add(s.a.y[b], 8); add(s.a.z[b], 8);
+            add(s.a.ox[b], 4); add(s.a.oy[b], 4); add(s.a.oz[b], 4);
+            add(s.a.cell[b], 4);
+        }
+        for (void *v : {s.a.px, s.a.py, s.a.pz, s.a.w, s.a.sx, s.a.sy, s.a.sz}) add(v, rs);
+        add(s.a.id, 4);
+        if (s.vs && s.sorted) {
+            a.vsink = vis_sink_of(c, s);
+            a.offs = s.offs;
+            a.keys_per_tile = c->keys_per_tile;
+        }
+        n = std::max<long long>(n, s.n_host);
+    }
+    if (!ns) return;
+    const unsigned blocks = (unsigned)((n + 255) / 256), few = std::min(blocks, 148u * 2u);
+    if (dead) {   // adjoint mode: particle indices must stay stable across steps
         prof_begin(c, "mark_dead");
-        mark_dead_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(a, s.dead);
+        mark_dead_kernel<<<dim3(blocks, ns), 256, 0, c->stream>>>(r);
         prof_end(c);
         return;
     }
     prof_begin(c, "remove_particles");
-    RemoveArgs a{};
-    a.g = g;
-    a.cp = c->cp;
-    a.fp32 = c->fp32;
-    a.count = s.d_count;
-    a.ctr = c->d_scratch_ll;
-    a.holes = c->d_list;
-    a.movers = c->d_list + c->list_cap / 2;
-    int cu = s.cur;
-    a.x = s.a.x[cu]; a.y = s.a.y[cu]; a.z = s.a.z[cu];
-    a.cell = s.a.cell[cu];
-    a.ox = s.a.ox[cu]; a.oy = s.a.oy[cu]; a.oz = s.a.oz[cu];
-    cudaMemsetAsync(c->d_scratch_ll, 0, 3 * sizeof(long long), c->stream);
-    unsigned blocks = (unsigned)((n + 255) / 256);
-    count_dead_kernel<<<blocks, 256, 0, c->stream>>>(a);
-    list_moves_kernel<<<blocks, 256, 0, c->stream>>>(a);
-    MoveArgs m{};
-    m.ctr = a.ctr;
-    m.count = s.d_count;
-    m.holes = a.holes;
-    m.movers = a.movers;
-    int k = 0, kf = 0;
-    for (int b = 0; b < 2; ++b) {
-        if (c->fp32) {
-            m.f[kf++] = s.a.ox[b]; m.f[kf++] = s.a.oy[b]; m.f[kf++] = s.a.oz[b];
-        } else {
-            m.d[k++] = s.a.x[b]; m.d[k++] = s.a.y[b]; m.d[k++] = s.a.z[b];
-        }
-    }
-    void *mom[7] = {s.a.px, s.a.py, s.a.pz, s.a.w, s.a.sx, s.a.sy, s.a.sz};
-    for (void *v : mom) {
-        if (!v) continue;
-        if (c->fp32) m.f[kf++] = (float *)v; else m.d[k++] = (double *)v;
-    }
-    m.i[0] = s.a.id;
-    m.i[1] = s.a.cell[0];
-    m.i[2] = s.a.cell[1];
-    (void)k;
-    if (s.vs && s.sorted) {
-        m.vsink = vis_sink_of(c, s);
-        m.at = a;
-        m.offs = s.offs;
-        m.keys_per_tile = c->keys_per_tile;
-        vis_drop_kernel<<<148 * 4, 256, 0, c->stream>>>(a, s.vraw, s.vs, s.vcap);
-    }
-    apply_moves_kernel<<<blocks, 256, 0, c->stream>>>(m);
-    finish_remove_kernel<<<1, 1, 0, c->stream>>>(s.d_count, c->d_scratch_ll);
+    cudaMemsetAsync(ctr, 0, 6 * sizeof(long long), c->stream);
+    list_dead_kernel<<<dim3(blocks, ns), 256, 0, c->stream>>>(r);
+    list_moves_kernel<<<dim3(few, ns), 256, 0, c->stream>>>(r);
+    apply_moves_kernel<<<dim3(few, ns), 256, 0, c->stream>>>(r);
     prof_end(c);
 }
 

@@ -116,7 +116,6 @@ int alloc_species(pic_ctx *c, int kind, int64_t cap, bool spin) {
     if (c->tile > 0 && cap > 0) {
         r = r ? r : alloc_arrays(c, s.b, n, spin);
         r = r ? r : dalloc(c, &s.keys, n * sizeof(int));
-        r = r ? r : dalloc(c, &s.strag, 2 * n * sizeof(int));
         r = r ? r : dalloc(c, &s.offs, (size_t)(c->nkeys + 1) * sizeof(unsigned));
         if (!c->p.adjoint) {
             // visitor lists for half of the capacity (a full list only makes
@@ -125,11 +124,12 @@ int alloc_species(pic_ctx *c, int kind, int64_t cap, bool spin) {
             s.vcap = (int64_t)(n / 2 + 1024);
             r = r ? r : dalloc(c, &s.vraw, 3 * (size_t)s.vcap * sizeof(int));
             r = r ? r : dalloc(c, &s.vis, 2 * (size_t)s.vcap * sizeof(int));
-            r = r ? r : dalloc(c, &s.vis_off, (nt + 1) * sizeof(unsigned));
-            r = r ? r : dalloc(c, &s.vis_cnt, (nt + 1) * sizeof(unsigned));
+            r = r ? r : dalloc(c, &s.vis_off, nt * sizeof(uint2));
+            r = r ? r : dalloc(c, &s.vis_cnt, nt * sizeof(unsigned));
             r = r ? r : dalloc(c, &s.vs, sizeof(VisState));
         }
     }
+    if (cap > 0) r = r ? r : dalloc(c, &s.strag, 2 * n * sizeof(int));
     r = r ? r : dalloc(c, &s.d_count, sizeof(long long));
     if (c->p.adjoint && cap > 0) r = r ? r : dalloc(c, &s.dead, n);
     if (c->p.adjoint && c->tile > 0 && cap > 0) {
@@ -144,7 +144,10 @@ int alloc_species(pic_ctx *c, int kind, int64_t cap, bool spin) {
     }
     cudaMemsetAsync(s.d_count, 0, sizeof(long long), c->stream);
     if (s.dead) cudaMemsetAsync(s.dead, 0, n, c->stream);
-    if (s.vs) cudaMemsetAsync(s.vs, 0, sizeof(VisState), c->stream);
+    if (s.vs) {
+        cudaMemsetAsync(s.vs, 0, sizeof(VisState), c->stream);
+        cudaMemsetAsync(s.vis_cnt, 0, (size_t)c->ntile[0] * c->ntile[1] * c->ntile[2] * sizeof(unsigned), c->stream);
+    }
     return PIC_OK;
 }
 
@@ -155,16 +158,6 @@ int ensure_stage(pic_ctx *c, size_t bytes) {
     c->stage_bytes = 0;
     int r = dalloc(c, (char **)&c->d_stage, bytes);
     if (r == PIC_OK) c->stage_bytes = bytes;
-    return r;
-}
-
-int ensure_lists(pic_ctx *c, int64_t n) {
-    if (c->list_cap >= 2 * n) return PIC_OK;
-    if (c->d_list) cudaFree(c->d_list);
-    c->d_list = nullptr;
-    c->list_cap = 0;
-    int r = dalloc(c, &c->d_list, (size_t)(2 * n) * sizeof(int));
-    if (r == PIC_OK) c->list_cap = 2 * n;
     return r;
 }
 
@@ -381,7 +374,7 @@ int begin_fill(pic_ctx *c, int kind, int64_t n, bool spin_nonzero, double wmax) 
     return ensure_stage(c, (size_t)(n < kChunk ? n : kChunk) * 144);
 }
 
-// the count of a filled species, and the compaction lists sized for it
+// the count of a filled species
 int end_fill(pic_ctx *c, int kind, int64_t n, const char *what) {
     Species &s = c->sp[kind];
     long long cnt = n;
@@ -389,8 +382,6 @@ int end_fill(pic_ctx *c, int kind, int64_t n, const char *what) {
     if (s.orig && n > 0) launch_iota(c, s.orig, n);   // upload index of every particle
     CK(cudaStreamSynchronize(c->stream));
     s.n_host = n;
-    int r = ensure_lists(c, n > c->sp[1 - kind].cap ? n : c->sp[1 - kind].cap);
-    if (r) return r;
     return launch_check(c, what);
 }
 
@@ -560,11 +551,12 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     for (int k = 0; k < 6 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->field[k], (size_t)c->g.fsz * rs);
     for (int k = 0; k < 5 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->ring[k], ((size_t)c->g.rsz * rs + 15) / 16 * 16);
     r = r ? r : dalloc(c, &c->d_status, sizeof(unsigned));
-    r = r ? r : dalloc(c, &c->d_scratch_ll, 8 * sizeof(long long));
+    r = r ? r : dalloc(c, &c->d_scratch_ll, 16 * sizeof(long long));
     r = r ? r : dalloc(c, &c->d_diag, PIC_NDIAG * sizeof(double));
     if (c->tile > 0) {
-        r = r ? r : dalloc(c, &c->d_hist, (size_t)(c->nkeys + 1) * sizeof(unsigned));
-        r = r ? r : dalloc(c, &c->d_blocksums, (size_t)(c->nkeys / 4096 + 2) * sizeof(unsigned));
+        c->sort_slots = sort_slots(c->nkeys);
+        r = r ? r : dalloc(c, &c->d_hist, sort_hist_bytes(c));
+        r = r ? r : dalloc(c, &c->d_blocksums, sort_sums_bytes(c));
         r = r ? r : dalloc(c, &c->d_nstrag, 2 * sizeof(unsigned long long));
     }
     if (r != PIC_OK) {
@@ -575,6 +567,10 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     for (int k = 0; k < 6; ++k) cudaMemsetAsync(c->field[k], 0, (size_t)c->g.fsz * rs, c->stream);
     for (int k = 0; k < 5; ++k) cudaMemsetAsync(c->ring[k], 0, (size_t)c->g.rsz * rs, c->stream);
     cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream);
+    if (c->tile > 0) {
+        cudaMemsetAsync(c->d_hist, 0, sort_hist_bytes(c), c->stream);
+        cudaMemsetAsync(c->d_blocksums, 0, sort_sums_bytes(c), c->stream);
+    }
     for (int k = 0; k < 2; ++k) {
         r = alloc_species(c, k, pp->capacity[k] > 0 ? pp->capacity[k] : 0, p.spin && p.mass[k] == 1.0);
         if (r != PIC_OK) {
@@ -609,7 +605,7 @@ int pic_destroy(pic_ctx *c) {
         if (c->h_pin[b]) cudaFreeHost(c->h_pin[b]);
         if (c->pin_ev[b]) cudaEventDestroy(c->pin_ev[b]);
     }
-    void *ptrs[] = {c->d_status, c->d_gtab, c->d_profile, c->d_stage, c->d_scratch_ll, c->d_list, c->d_diag,
+    void *ptrs[] = {c->d_status, c->d_gtab, c->d_profile, c->d_stage, c->d_scratch_ll, c->d_diag,
                     c->d_hist, c->d_blocksums, c->d_nstrag};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -958,7 +954,7 @@ static int push_both(pic_ctx *c) {
 
 int pic_exchange_particles(pic_ctx *c, int kind) {
     if (!c || kind < 0 || kind > 1) return PIC_EINVAL;
-    if (c->sp[kind].n_host > 0) launch_remove(c, kind);
+    launch_remove(c, 1 << kind);
     return launch_check(c, "exchange_particles");
 }
 
@@ -1039,8 +1035,8 @@ int pic_initial_push(pic_ctx *c) {
     launch_sort_due(c, 3);   // before the tape records the particles: the push runs in sorted order
     adjoint_record_hook(c);
     if ((r = push_both(c))) return r;
-    if ((r = pic_exchange_particles(c, 0))) return r;
-    return pic_exchange_particles(c, 1);
+    launch_remove(c, 3);
+    return launch_check(c, "exchange_particles");
 }
 
 // One iteration of run_main_time_loop.  rho (a diagnostic: it never feeds
@@ -1061,8 +1057,8 @@ static int run_one_step(pic_ctx *c, bool rho_observed, bool e_first, bool e_next
     launch_sort_due(c, 3);
     adjoint_record_hook(c);
     if ((r = push_both(c))) return r;
-    if ((r = pic_exchange_particles(c, 0))) return r;
-    if ((r = pic_exchange_particles(c, 1))) return r;
+    launch_remove(c, 3);
+    if ((r = launch_check(c, "exchange_particles"))) return r;
     launch_update_b_fold(c, c->p.dt_half, rings);
     launch_update_e(c, c->p.dt_half, e_next);
     return launch_check(c, "update_fields_second");

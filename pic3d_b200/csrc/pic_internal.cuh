@@ -106,23 +106,28 @@ struct PartArrays {
 // half-cell octants per cell in the particle sort key (tile, octant, cell)
 constexpr int kOctants = 8;
 
-// Visitor-list state of one species on the device.  valid_cur: the lists
-// the running push reads name every particle that is away from its home
-// tile (else the push falls back to handing such particles to the global
-// kernel).  valid_next: the same for the entries the running push appends;
-// cleared when vraw overflows, when removal compacts the arrays, or when a
-// particle lands outside the tile grid on a periodic axis.
+// Visitor-list state of one species on the device.  A push appends its
+// entries under one of two counters, chosen by the host's parity
+// (Species::vis_par); building the lists from them starts the other one.
+// valid_cur: the lists the running push reads name every particle that is
+// away from its home tile (else the push falls back to handing such particles
+// to the global kernel).  valid_next: the same for the entries the running
+// push appends; cleared when vraw overflows or when a particle lands outside
+// the tile grid on a periodic axis.
 struct VisState {
-    unsigned long long nraw;   // entries appended to vraw by the running push
-    unsigned valid_cur, valid_next;
-    unsigned long long nvis;   // entries of the current lists
+    unsigned long long nraw[2];   // entries appended to vraw
+    unsigned valid_next[2], valid_cur;
+    unsigned total;               // slots handed out while the lists are built
+    unsigned long long nvis;      // entries of the current lists
 };
 
 // Where a push records the particles that end away from their home tile
 // (raw null: not recorded).  See Species::vraw.
 struct VisSink {
     int *raw;                    // (index, home tile, new tile) triples
-    VisState *vs;
+    unsigned long long *nraw;    // counters and flag of the push's parity (VisState)
+    unsigned *valid;
+    unsigned *cnt;               // entries per new tile
     long long cap;               // triples
     int T, nt[3];
     int nodes;                   // 1: tiles hold nodes (pic_ctx::node_tiles), 0: cells
@@ -136,19 +141,24 @@ struct Species {
     PartArrays a;            // the particles
     PartArrays b;            // destination of the counting sort (same shapes)
     int *keys = nullptr;     // per-particle sort key
-    int *strag = nullptr;    // particles the tiled kernel hands to the global kernel: (index, home tile) pairs
+    // particles the tiled kernel hands to the global kernel, (index, home
+    // tile) pairs; between pushes the index lists of the removal
+    int *strag = nullptr;
+    bool strag_zero = false;   // the straggler count has been cleared for the next push
     // Incremental re-binning between full sorts.  A particle's home tile is
     // the tile whose slice of the sorted arrays holds it; a particle whose
     // cell lies in another tile is a visitor there.  Each push appends
     // (index, home, new tile) for every particle that ends away from home
-    // (vraw); before the next push a counting sort of those entries by tile
-    // gives each tile its visitor list (vis, (index, home) pairs, vis_off).
+    // (vraw) and counts it under its new tile (vis_cnt); before the next push
+    // each tile is given a range of the visitor list (vis_off) and the entries
+    // are scattered to them (vis, (index, home) pairs).
     int *vraw = nullptr;
     int *vis = nullptr;
-    unsigned *vis_off = nullptr;   // ntiles + 1
-    unsigned *vis_cnt = nullptr;   // ntiles + 1 (histogram, then cursor)
+    uint2 *vis_off = nullptr;      // per tile: begin and end of its visitors
+    unsigned *vis_cnt = nullptr;   // per tile; zero once the lists are built
     int64_t vcap = 0;              // entries of vraw / vis
     VisState *vs = nullptr;        // device counters and flags
+    int vis_par = 0;               // VisState counter the coming push records under
     int vis_built_for = -1;        // pushes_since_sort when the lists were last built
     unsigned char *dead = nullptr;  // adjoint mode: 1 once a particle left through an absorbing face
     // adjoint mode with tiles: the sort moves every per-particle array, so
@@ -208,8 +218,6 @@ struct pic_ctx {
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
     long long *d_scratch_ll = nullptr;   // small counters
-    int *d_list = nullptr;               // compaction index lists
-    int64_t list_cap = 0;
     double *d_diag = nullptr;
     // pinned host staging for particle uploads / downloads: two buffers of
     // kPinRecords records each, used alternately so that the host copy of
@@ -226,8 +234,12 @@ struct pic_ctx {
     bool node_tiles = false;
     long long keys_per_tile = 0;         // tile^3 (nodes) or kOctants * tile^3 (cells)
     long long nkeys = 0;                 // ntiles * keys_per_tile
-    unsigned *d_hist = nullptr;          // nkeys + 1
-    unsigned *d_blocksums = nullptr;
+    // key histograms (zero between sorts) and their scan's block sums.  Two
+    // slots, so that both species sort in the same launches, while the second
+    // is small (kSortSlotKeys): on large grids the launches do not matter.
+    unsigned *d_hist = nullptr;          // sort_slots x nkeys
+    unsigned *d_blocksums = nullptr;     // sort_slots x (blocks + 1), then the count of finished blocks
+    int sort_slots = 1;
     unsigned long long *d_nstrag = nullptr;   // straggler counts, one per species
     int sort_interval = 4;
     // rho is observable only between ABI calls: the intermediate steps of

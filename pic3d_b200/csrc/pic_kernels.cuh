@@ -44,9 +44,8 @@ struct ThermalArgs {
 void launch_lattice_records(pic_ctx *c, const LatticeArgs &a);
 void launch_thermal_records(pic_ctx *c, const ThermalArgs &a);
 void launch_push(pic_ctx *c, int kind);
-// idx: (index, home tile) pairs; visitors recorded into v when v.raw is set
-void launch_push_list(pic_ctx *c, int kind, const int *idx, const unsigned long long *count, const VisSink &v);
-void launch_remove(pic_ctx *c, int kind);
+void launch_push_stragglers(pic_ctx *c, int mask);   // the particles the tile kernel left, both species in one launch
+void launch_remove(pic_ctx *c, int mask);
 void launch_upload_particles(pic_ctx *c, int kind, const void *d_records, int64_t n, int64_t offset,
                              unsigned long long *check = nullptr);
 void launch_download_particles(pic_ctx *c, int kind, void *d_records, int64_t n, int64_t offset);
@@ -55,9 +54,11 @@ void launch_iota(pic_ctx *c, int *a, long long n);   // a[i] = i
 void launch_deposit_one(pic_ctx *c, int kind, const double (&xo)[3], const double (&xn)[3], double qw);
 
 // tile_kernels.cu
-void launch_sort(pic_ctx *c, int kind);
 void launch_sort_due(pic_ctx *c, int mask);   // the sorts the next push of the masked species needs
 void launch_tile_push(pic_ctx *c, int mask);
+int sort_slots(long long nkeys);              // histograms a context keeps (pic_ctx::sort_slots)
+size_t sort_hist_bytes(const pic_ctx *c);
+size_t sort_sums_bytes(const pic_ctx *c);
 int tile_order_stats(pic_ctx *c, int kind, long long (&out)[4]);
 VisSink vis_sink_of(const pic_ctx *c, const Species &s);   // where a push of species s records visitors
 // Row and plane strides of a tile kernel's shared box of extent e for tile

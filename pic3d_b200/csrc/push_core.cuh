@@ -43,17 +43,18 @@ __device__ __forceinline__ void vis_note(const VisSink &v, const Geom &g, int p,
             per_out = per_out || (o && g.per[d]);
         }
         if (!in) {
-            if (per_out) v.vs->valid_next = 0u;
+            if (per_out) *v.valid = 0u;
             return;
         }
         t = ((cell[2] / v.T) * v.nt[1] + cell[1] / v.T) * v.nt[0] + cell[0] / v.T;
         if (t == home) return;
     }
-    const unsigned long long s = atomicAdd(&v.vs->nraw, 1ull);
+    const unsigned long long s = atomicAdd(v.nraw, 1ull);
     if ((long long)s >= v.cap) {
-        v.vs->valid_next = 0u;
+        *v.valid = 0u;
         return;
     }
+    atomicAdd(v.cnt + t, 1u);
     v.raw[3 * s] = p;
     v.raw[3 * s + 1] = home;
     v.raw[3 * s + 2] = t;

@@ -63,7 +63,7 @@ struct TileArgs {
     // visitor lists of this push (vis_off null: none) and the recording of
     // the next push's (vsink.raw null: off)
     const int *vis[2];
-    const unsigned *vis_off[2];
+    const uint2 *vis_off[2];
     const VisState *vs[2];
     VisSink vsink[2];
 };

@@ -20,7 +20,8 @@
 // shared-memory addresses fall in different banks.
 //
 // The counting sort (key histogram, exclusive scan, scatter into the second
-// set of arrays) runs every `sort_interval` pushes and after an upload.
+// set of arrays) runs every `sort_interval` pushes and after an upload; one
+// set of launches sorts both species.
 #include "tile_common.cuh"
 
 namespace pic {
@@ -83,148 +84,188 @@ __device__ __forceinline__ int particle_key(const Geom &g, const TileGeom &t, co
 }
 
 // ---------------------------------------------------------------------------
-// counting sort
+// counting sort.  One launch of each kernel serves up to two species
+// (blockIdx.y): a 32^3 step is bound by launches and the gaps between them,
+// about 2.3 us each.
+
+constexpr int kSortKeysPerBlock = 4096;   // of the scan, 4 per thread
 
 struct SortArgs {
     Geom g;
     TileGeom t;
     CellPack cp;
     int fp32;
-    const long long *count;
-    const double *x, *y, *z;
-    const int *cell;
-    const float *ox, *oy, *oz;
-    int *keys;
-    unsigned *hist;
+    unsigned *done;              // blocks of the scan that have finished, per species (zero between sorts)
+    int ntiles;
+    struct One {
+        const long long *count;
+        const double *x, *y, *z;
+        const int *cell;
+        const float *ox, *oy, *oz;
+        int *keys;
+        unsigned *hist, *sums, *offs;
+        // visitor lists (null: none) and the straggler count, reset here
+        VisState *vs;
+        int par;
+        uint2 *vis_off;
+        unsigned *vis_cnt;
+        unsigned long long *nstrag;
+    } s[2];
 };
 
-__global__ void sort_keys_kernel(SortArgs a) {
+__global__ void sort_keys_kernel(const __grid_constant__ SortArgs sa) {
+    const SortArgs::One &a = sa.s[blockIdx.y];
     long long n = *a.count;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned act = __ballot_sync(0xffffffffu, i < n);
     if (i >= n) return;
-    int key = particle_key(a.g, a.t, a.cp, a.fp32, a.x, a.y, a.z, a.cell, a.ox, a.oy, a.oz, i);
+    int key = particle_key(sa.g, sa.t, sa.cp, sa.fp32, a.x, a.y, a.z, a.cell, a.ox, a.oy, a.oz, i);
     a.keys[i] = key;
     unsigned peers = __match_any_sync(act, key);
     int lane = threadIdx.x & 31;
     if (lane == __ffs(peers) - 1) atomicAdd(&a.hist[key], (unsigned)__popc(peers));
 }
 
-// exclusive scan of n unsigned values in place; block sums in `sums`
-__global__ void scan_blocks_kernel(unsigned *v, long long n, unsigned *sums) {
-    __shared__ unsigned warp_tot[32];
-    const int per = 4;
-    long long base = (long long)blockIdx.x * blockDim.x * per + (long long)threadIdx.x * per;
-    unsigned loc[per];
-    unsigned s = 0;
-#pragma unroll
-    for (int k = 0; k < per; ++k) {
-        loc[k] = base + k < n ? v[base + k] : 0u;
-        s += loc[k];
-    }
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// exclusive sum over the block (1024 threads) of one value per thread;
+// `total` gets the block's sum
+__device__ __forceinline__ unsigned block_exclusive(unsigned s, unsigned &total) {
+    __shared__ unsigned warp_tot[33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned incl = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+        const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += t;
     }
     if (lane == 31) warp_tot[w] = incl;
     __syncthreads();
     if (w == 0) {
-        int nw = blockDim.x >> 5;
-        unsigned t = lane < nw ? warp_tot[lane] : 0u;
+        const int nw = blockDim.x >> 5;
+        const unsigned t = lane < nw ? warp_tot[lane] : 0u;
         unsigned ti = t;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            unsigned u = __shfl_up_sync(0xffffffffu, ti, o);
+            const unsigned u = __shfl_up_sync(0xffffffffu, ti, o);
             if (lane >= o) ti += u;
         }
         if (lane < nw) warp_tot[lane] = ti - t;
-        if (lane == nw - 1) sums[blockIdx.x] = ti;
+        if (lane == nw - 1) warp_tot[32] = ti;
     }
     __syncthreads();
-    unsigned run = warp_tot[w] + incl - s;
+    const unsigned excl = warp_tot[w] + incl - s;
+    total = warp_tot[32];
+    __syncthreads();
+    return excl;
+}
+
+// Sums of the histogram's blocks of kSortKeysPerBlock keys; the last block to
+// finish turns them into exclusive offsets (sums[nb]: the total), so that the
+// scan takes two launches.  Every particle is at home after the sort: the
+// visitor lists are emptied, the straggler count too.
+__global__ void __launch_bounds__(1024) sort_sums_kernel(const __grid_constant__ SortArgs sa, int nb) {
+    const SortArgs::One &a = sa.s[blockIdx.y];
+    __shared__ bool last;
+    const long long base = (long long)blockIdx.x * kSortKeysPerBlock + (long long)threadIdx.x * 4;
+    unsigned s = 0;
 #pragma unroll
-    for (int k = 0; k < per; ++k) {
-        if (base + k < n) v[base + k] = run;
+    for (int k = 0; k < 4; ++k) s += base + k < sa.t.nkeys ? a.hist[base + k] : 0u;
+    unsigned total;
+    block_exclusive(s, total);
+    if (threadIdx.x == 0) {
+        a.sums[blockIdx.x] = total;
+        __threadfence();
+        last = atomicAdd(sa.done + blockIdx.y, 1u) == gridDim.x - 1;
+    }
+    if (a.vs) {
+        for (int q = blockIdx.x * 1024 + threadIdx.x; q < sa.ntiles; q += gridDim.x * 1024) {
+            a.vis_off[q] = make_uint2(0u, 0u);
+            a.vis_cnt[q] = 0u;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    unsigned carry = 0;
+    for (int off = 0; off < nb; off += 1024) {
+        const int i = off + threadIdx.x;
+        const unsigned v = i < nb ? __ldcg(a.sums + i) : 0u;
+        const unsigned e = block_exclusive(v, total);
+        if (i < nb) a.sums[i] = carry + e;
+        carry += total;
+    }
+    if (threadIdx.x == 0) {
+        a.sums[nb] = carry;
+        sa.done[blockIdx.y] = 0u;
+        *a.nstrag = 0ull;
+        if (a.vs) {
+            a.vs->nraw[a.par] = 0ull;
+            a.vs->valid_next[a.par] = 1u;
+            a.vs->valid_cur = 1u;
+            a.vs->total = 0u;
+            a.vs->nvis = 0ull;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(1024) sort_offsets_kernel(const __grid_constant__ SortArgs sa, int nb) {
+    const SortArgs::One &a = sa.s[blockIdx.y];
+    const long long base = (long long)blockIdx.x * kSortKeysPerBlock + (long long)threadIdx.x * 4;
+    unsigned loc[4], s = 0, total;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        loc[k] = base + k < sa.t.nkeys ? a.hist[base + k] : 0u;
+        s += loc[k];
+    }
+    unsigned run = block_exclusive(s, total) + a.sums[blockIdx.x];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (base + k < sa.t.nkeys) a.offs[base + k] = run;
         run += loc[k];
     }
-}
-
-// exclusive scan of the block sums (single block, any count), total in sums[nb]
-__global__ void scan_sums_kernel(unsigned *sums, int nb) {
-    __shared__ unsigned carry;
-    __shared__ unsigned warp_tot[32];
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int off = 0; off < nb; off += blockDim.x) {
-        int i = off + threadIdx.x;
-        unsigned s = i < nb ? sums[i] : 0u;
-        int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        unsigned incl = s;
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) warp_tot[w] = incl;
-        __syncthreads();
-        if (w == 0) {
-            int nw = blockDim.x >> 5;
-            unsigned t = lane < nw ? warp_tot[lane] : 0u;
-            unsigned ti = t;
-            for (int o = 1; o < 32; o <<= 1) {
-                unsigned u = __shfl_up_sync(0xffffffffu, ti, o);
-                if (lane >= o) ti += u;
-            }
-            if (lane < nw) warp_tot[lane] = ti - t;
-        }
-        __syncthreads();
-        unsigned excl = carry + warp_tot[w] + incl - s;
-        if (i < nb) sums[i] = excl;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = excl + s;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) sums[nb] = carry;
-}
-
-__global__ void scan_add_kernel(unsigned *v, long long n, const unsigned *sums, int per_block, unsigned *offs_out,
-                                unsigned *cursor_out) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        unsigned o = v[i] + sums[i / per_block];
-        offs_out[i] = o;
-        cursor_out[i] = o;
-    }
-    if (i == n) {
-        int nb = (int)((n + per_block - 1) / per_block);
-        offs_out[n] = sums[nb];
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.offs[sa.t.nkeys] = a.sums[nb];
 }
 
 struct ScatterArgs {
-    const long long *count;
-    long long cap;
     unsigned *status;
-    const int *keys;
-    unsigned *cursor;
-    // up to 16 8-byte and 16 4-byte arrays moved src -> dst
-    const double *ds[16];
-    double *dd[16];
-    int nd;
-    const float *fs[16];
-    float *fd[16];
-    int nf;
-    const int *is[4];
-    int *id_[4];
-    int ni;
-    const unsigned char *bs;   // one byte array (adjoint mode: dead flags), or null
-    unsigned char *bd;
-    int *perm;                 // adjoint mode: perm[dst] = src, the gather form of this sort
+    struct One {
+        const long long *count;
+        long long cap;
+        const int *keys;
+        const unsigned *offs;
+        unsigned *hist;            // counted down to zero: the next sort's histogram
+        // arrays moved src -> dst: at most 13 of 8 bytes (two position buffers,
+        // momenta, weight, spins) and 17 of 4 (the same in FP32, id, upload index)
+        const double *ds[13];
+        double *dd[13];
+        int nd;
+        const unsigned *fs[17];
+        unsigned *fd[17];
+        int nf;
+        const unsigned char *bs;   // one byte array (adjoint mode: dead flags), or null
+        unsigned char *bd;
+        int *perm;                 // adjoint mode: perm[dst] = src, the gather form of this sort
+    } s[2];
 };
 
-__global__ void scatter_kernel(ScatterArgs a) {
+// moves element i of n arrays to dst, the loads of eight arrays before their
+// stores (the compiler must assume that a store changes the next source)
+template <typename T, int N>
+__device__ __forceinline__ void move_words(const T *const (&src)[N], T *const (&to)[N], int n, long long i, unsigned dst) {
+#pragma unroll
+    for (int k0 = 0; k0 < N; k0 += 8) {
+        if (k0 >= n) break;
+        T v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < N && k0 + k < n) v[k] = src[k0 + k][i];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < N && k0 + k < n) to[k0 + k][dst] = v[k];
+    }
+}
+
+__global__ void __launch_bounds__(256) scatter_kernel(const __grid_constant__ ScatterArgs sa) {
+    const ScatterArgs::One &a = sa.s[blockIdx.y];
     long long n = *a.count;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned act = __ballot_sync(0xffffffffu, i < n);
@@ -234,47 +275,27 @@ __global__ void scatter_kernel(ScatterArgs a) {
     int lane = threadIdx.x & 31;
     int leader = __ffs(peers) - 1;
     unsigned base = 0;
-    if (lane == leader) base = atomicAdd(&a.cursor[key], (unsigned)__popc(peers));
+    if (lane == leader) {
+        const unsigned k = (unsigned)__popc(peers);
+        base = a.offs[key] + atomicSub(&a.hist[key], k) - k;
+    }
     base = __shfl_sync(peers, base, leader);
     unsigned dst = base + __popc(peers & ((1u << lane) - 1u));
     if ((long long)dst >= a.cap) {  // cannot happen with a consistent histogram; never write past the arrays
-        atomicOr(a.status, ST_OVERFLOW);
+        atomicOr(sa.status, ST_OVERFLOW);
         return;
     }
-    for (int k = 0; k < a.nd; ++k) a.dd[k][dst] = a.ds[k][i];
-    for (int k = 0; k < a.nf; ++k) a.fd[k][dst] = a.fs[k][i];
-    for (int k = 0; k < a.ni; ++k) a.id_[k][dst] = a.is[k][i];
+    move_words(a.ds, a.dd, a.nd, i, dst);
+    move_words(a.fs, a.fd, a.nf, i, dst);
     if (a.bs) a.bd[dst] = a.bs[i];
     if (a.perm) a.perm[dst] = (int)i;
 }
 
 // ---------------------------------------------------------------------------
 // visitor lists: a counting sort by tile of the (index, home, tile) entries
-// the last push recorded
-
-__global__ void vis_reset_kernel(VisState *vs) {
-    vs->nraw = 0;
-    vs->nvis = 0;
-    vs->valid_cur = 1u;
-    vs->valid_next = 1u;
-}
-
-// entries with tile -1 were dropped by the removal compaction
-__global__ void vis_hist_kernel(const int *raw, const VisState *vs, long long cap, unsigned *cnt) {
-    const long long n = min((long long)vs->nraw, cap);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        if (raw[3 * i + 2] >= 0) atomicAdd(&cnt[raw[3 * i + 2]], 1u);
-}
-
-__global__ void vis_scatter_kernel(const int *raw, const VisState *vs, long long cap, unsigned *cursor, int *vis) {
-    const long long n = min((long long)vs->nraw, cap);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        if (raw[3 * i + 2] < 0) continue;
-        const unsigned slot = atomicAdd(&cursor[raw[3 * i + 2]], 1u);
-        vis[2 * slot] = raw[3 * i];
-        vis[2 * slot + 1] = raw[3 * i + 1];
-    }
-}
+// the last push recorded (and counted under their tiles), in two launches:
+// each tile is given a range of the list, in no particular order of the
+// tiles, then the entries are scattered.
 
 // FP64: below this fraction of a species away from home, the particles away
 // from home are pushed by the global-memory kernel instead.  On the
@@ -290,28 +311,83 @@ __host__ __device__ inline bool visitor_lists_pay(unsigned long long entries, lo
     return (double)entries >= min_frac * (double)particles;
 }
 
-// the lists just built are the ones the coming push reads; it records into
-// an empty raw list
-__global__ void vis_rotate_kernel(VisState *vs, long long cap, const long long *count, double min_frac) {
-    vs->nvis = min((long long)vs->nraw, cap);
-    vs->valid_cur = vs->valid_next && visitor_lists_pay(vs->nvis, *count, min_frac);
-    vs->nraw = 0;
-    vs->valid_next = 1u;
+struct VisArgs {
+    int ntiles;
+    double min_frac;
+    struct One {
+        const long long *count;
+        const int *raw;
+        int *vis;
+        uint2 *off;
+        unsigned *cnt;
+        VisState *vs;
+        int par;                 // the counter the last push recorded under
+        long long cap;
+        unsigned long long *nstrag;
+    } s[2];
+};
+
+// The lists become the ones the coming push reads; it records under the
+// other counter.
+__global__ void __launch_bounds__(1024) vis_ranges_kernel(const __grid_constant__ VisArgs va) {
+    const VisArgs::One &a = va.s[blockIdx.y];
+    __shared__ unsigned first;
+    const int base = (int)(blockIdx.x * 4096 + threadIdx.x * 4);
+    unsigned loc[4], s = 0, total;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        loc[k] = base + k < va.ntiles ? a.cnt[base + k] : 0u;
+        s += loc[k];
+    }
+    unsigned run = block_exclusive(s, total);
+    if (threadIdx.x == 0) first = atomicAdd(&a.vs->total, total);
+    __syncthreads();
+    run += first;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (base + k < va.ntiles) a.off[base + k] = make_uint2(run, run + loc[k]);
+        run += loc[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        VisState &v = *a.vs;
+        v.nvis = min((long long)v.nraw[a.par], a.cap);
+        v.valid_cur = v.valid_next[a.par] && visitor_lists_pay(v.nvis, *a.count, va.min_frac);
+        v.nraw[a.par ^ 1] = 0ull;
+        v.valid_next[a.par ^ 1] = 1u;
+        *a.nstrag = 0ull;
+    }
 }
 
-static void launch_vis_build(pic_ctx *c, Species &s) {
-    const long long nt = (long long)c->ntile[0] * c->ntile[1] * c->ntile[2];
-    const int per_block = 1024 * 4;
-    const int sb = (int)((nt + per_block - 1) / per_block);
-    const unsigned grid = 148 * 4;
-    cudaMemsetAsync(s.vis_cnt, 0, (size_t)(nt + 1) * sizeof(unsigned), c->stream);
-    vis_hist_kernel<<<grid, 256, 0, c->stream>>>(s.vraw, s.vs, s.vcap, s.vis_cnt);
-    scan_blocks_kernel<<<sb, 1024, 0, c->stream>>>(s.vis_cnt, nt, c->d_blocksums);
-    scan_sums_kernel<<<1, 1024, 0, c->stream>>>(c->d_blocksums, sb);
-    scan_add_kernel<<<(unsigned)((nt + 1 + 255) / 256), 256, 0, c->stream>>>(s.vis_cnt, nt, c->d_blocksums, per_block,
-                                                                             s.vis_off, s.vis_cnt);
-    vis_scatter_kernel<<<grid, 256, 0, c->stream>>>(s.vraw, s.vs, s.vcap, s.vis_cnt, s.vis);
-    vis_rotate_kernel<<<1, 1, 0, c->stream>>>(s.vs, s.vcap, s.d_count, visitor_min_fraction(c));
+// entries with tile -1 were dropped by the removal compaction
+__global__ void __launch_bounds__(256) vis_scatter_kernel(const __grid_constant__ VisArgs va) {
+    const VisArgs::One &a = va.s[blockIdx.y];
+    const long long n = min((long long)a.vs->nraw[a.par], a.cap);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const int p = a.raw[3 * i], home = a.raw[3 * i + 1], t = a.raw[3 * i + 2];
+        if (t < 0) continue;
+        const unsigned slot = a.off[t].x + atomicSub(a.cnt + t, 1u) - 1u;
+        reinterpret_cast<int2 *>(a.vis)[slot] = make_int2(p, home);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.vs->total = 0u;
+}
+
+static void launch_vis_build(pic_ctx *c, int mask) {
+    VisArgs va{};
+    va.ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
+    va.min_frac = visitor_min_fraction(c);
+    unsigned ns = 0;
+    long long n = 0;
+    for (int k = 0; k < 2; ++k) {
+        if (!((mask >> k) & 1)) continue;
+        Species &s = c->sp[k];
+        va.s[ns++] = VisArgs::One{s.d_count, s.vraw, s.vis, s.vis_off, s.vis_cnt, s.vs, s.vis_par, s.vcap, c->d_nstrag + k};
+        s.vis_par ^= 1;
+        s.strag_zero = true;
+        n = std::max<long long>(n, s.vcap);
+    }
+    vis_ranges_kernel<<<dim3((unsigned)((va.ntiles + 4095) / 4096), ns), 1024, 0, c->stream>>>(va);
+    const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 148 * 4);
+    vis_scatter_kernel<<<dim3(grid, ns), 256, 0, c->stream>>>(va);
 }
 
 static TileGeom tile_geom(const pic_ctx *c) {
@@ -323,110 +399,156 @@ static TileGeom tile_geom(const pic_ctx *c) {
     return t;
 }
 
-void launch_sort(pic_ctx *c, int kind) {
-    Species &s = c->sp[kind];
-    const long long n = s.n_host;
-    if (n <= 0 || c->tile <= 0) return;
-    prof_begin(c, "sort_particles");
-    const long long K = c->nkeys;
-    cudaMemsetAsync(c->d_hist, 0, (size_t)(K + 1) * sizeof(unsigned), c->stream);
+int sort_slots(long long nkeys) { return nkeys <= (1ll << 24) ? 2 : 1; }
+size_t sort_hist_bytes(const pic_ctx *c) { return (size_t)c->sort_slots * c->nkeys * sizeof(unsigned); }
+static int scan_blocks(const pic_ctx *c) { return (int)((c->nkeys + kSortKeysPerBlock - 1) / kSortKeysPerBlock); }
+size_t sort_sums_bytes(const pic_ctx *c) {
+    return ((size_t)c->sort_slots * (scan_blocks(c) + 1) + 2) * sizeof(unsigned);
+}
+
+// the species of `mask` (all with particles), in one set of launches
+static void sort_together(pic_ctx *c, int mask) {
+    const int sb = scan_blocks(c);
     SortArgs a{};
+    ScatterArgs sa{};
     a.g = c->g;
     a.t = tile_geom(c);
     a.cp = c->cp;
     a.fp32 = c->fp32;
-    a.count = s.d_count;
-    a.x = s.a.x[s.cur]; a.y = s.a.y[s.cur]; a.z = s.a.z[s.cur];
-    a.cell = s.a.cell[s.cur];
-    a.ox = s.a.ox[s.cur]; a.oy = s.a.oy[s.cur]; a.oz = s.a.oz[s.cur];
-    a.keys = s.keys;
-    a.hist = c->d_hist;
-    unsigned nb = (unsigned)((n + 255) / 256);
-    sort_keys_kernel<<<nb, 256, 0, c->stream>>>(a);
-    const int per_block = 1024 * 4;
-    int sb = (int)((K + per_block - 1) / per_block);
-    scan_blocks_kernel<<<sb, 1024, 0, c->stream>>>(c->d_hist, K, c->d_blocksums);
-    scan_sums_kernel<<<1, 1024, 0, c->stream>>>(c->d_blocksums, sb);
-    // offsets into s.offs; the cursor reuses d_hist
-    scan_add_kernel<<<(unsigned)((K + 1 + 255) / 256), 256, 0, c->stream>>>(c->d_hist, K, c->d_blocksums,
-                                                                            per_block, s.offs, c->d_hist);
-    ScatterArgs sa{};
-    sa.count = s.d_count;
-    sa.cap = s.cap;
+    a.ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
+    a.done = c->d_blocksums + (size_t)c->sort_slots * (sb + 1);
     sa.status = c->d_status;
-    sa.keys = s.keys;
-    sa.cursor = c->d_hist;
-    // The sort runs right before a push, which overwrites the previous-position
-    // buffer: only the current one moves (the adjoint's tape keeps both).
-    for (int b = 0; b < 2; ++b) {
-        if (b != s.cur && !c->p.adjoint) continue;
-        if (c->fp32) {
-            sa.fs[sa.nf] = s.a.ox[b]; sa.fd[sa.nf++] = s.b.ox[b];
-            sa.fs[sa.nf] = s.a.oy[b]; sa.fd[sa.nf++] = s.b.oy[b];
-            sa.fs[sa.nf] = s.a.oz[b]; sa.fd[sa.nf++] = s.b.oz[b];
-            sa.is[sa.ni] = s.a.cell[b]; sa.id_[sa.ni++] = s.b.cell[b];
-        } else {
-            sa.ds[sa.nd] = s.a.x[b]; sa.dd[sa.nd++] = s.b.x[b];
-            sa.ds[sa.nd] = s.a.y[b]; sa.dd[sa.nd++] = s.b.y[b];
-            sa.ds[sa.nd] = s.a.z[b]; sa.dd[sa.nd++] = s.b.z[b];
+    unsigned ns = 0;
+    long long nmax = 0;
+    for (int kind = 0; kind < 2; ++kind) {
+        if (!((mask >> kind) & 1)) continue;
+        Species &s = c->sp[kind];
+        SortArgs::One &o = a.s[ns];
+        o.count = s.d_count;
+        o.x = s.a.x[s.cur]; o.y = s.a.y[s.cur]; o.z = s.a.z[s.cur];
+        o.cell = s.a.cell[s.cur];
+        o.ox = s.a.ox[s.cur]; o.oy = s.a.oy[s.cur]; o.oz = s.a.oz[s.cur];
+        o.keys = s.keys;
+        o.hist = c->d_hist + (size_t)ns * c->nkeys;
+        o.sums = c->d_blocksums + (size_t)ns * (sb + 1);
+        o.offs = s.offs;
+        o.vs = s.vs;
+        o.par = s.vis_par;
+        o.vis_off = s.vis_off;
+        o.vis_cnt = s.vis_cnt;
+        o.nstrag = c->d_nstrag + kind;
+        ScatterArgs::One &m = sa.s[ns++];
+        m.count = s.d_count;
+        m.cap = s.cap;
+        m.keys = s.keys;
+        m.offs = s.offs;
+        m.hist = o.hist;
+        auto word = [&](const void *src, void *dst) {
+            m.fs[m.nf] = (const unsigned *)src;
+            m.fd[m.nf++] = (unsigned *)dst;
+        };
+        auto dbl = [&](const void *src, void *dst) {
+            m.ds[m.nd] = (const double *)src;
+            m.dd[m.nd++] = (double *)dst;
+        };
+        // The sort runs right before a push, which overwrites the previous-position
+        // buffer: only the current one moves (the adjoint's tape keeps both).
+        for (int b = 0; b < 2; ++b) {
+            if (b != s.cur && !c->p.adjoint) continue;
+            if (c->fp32) {
+                word(s.a.ox[b], s.b.ox[b]);
+                word(s.a.oy[b], s.b.oy[b]);
+                word(s.a.oz[b], s.b.oz[b]);
+                word(s.a.cell[b], s.b.cell[b]);
+            } else {
+                dbl(s.a.x[b], s.b.x[b]);
+                dbl(s.a.y[b], s.b.y[b]);
+                dbl(s.a.z[b], s.b.z[b]);
+            }
         }
+        void *src[7] = {s.a.px, s.a.py, s.a.pz, s.a.w, s.a.sx, s.a.sy, s.a.sz};
+        void *dst[7] = {s.b.px, s.b.py, s.b.pz, s.b.w, s.b.sx, s.b.sy, s.b.sz};
+        for (int k = 0; k < 7; ++k) {
+            if (!src[k]) continue;
+            if (c->fp32) word(src[k], dst[k]);
+            else dbl(src[k], dst[k]);
+        }
+        word(s.a.id, s.b.id);
+        if (s.orig) {   // adjoint mode: upload index, dead flags, and the permutation for the tape
+            word(s.orig, s.orig_b);
+            m.bs = s.dead;
+            m.bd = s.dead_b;
+            m.perm = s.perm;
+        }
+        nmax = std::max<long long>(nmax, s.n_host);
     }
-    void *src[7] = {s.a.px, s.a.py, s.a.pz, s.a.w, s.a.sx, s.a.sy, s.a.sz};
-    void *dst[7] = {s.b.px, s.b.py, s.b.pz, s.b.w, s.b.sx, s.b.sy, s.b.sz};
-    for (int k = 0; k < 7; ++k) {
-        if (!src[k]) continue;
-        if (c->fp32) { sa.fs[sa.nf] = (float *)src[k]; sa.fd[sa.nf++] = (float *)dst[k]; }
-        else { sa.ds[sa.nd] = (double *)src[k]; sa.dd[sa.nd++] = (double *)dst[k]; }
+    const unsigned nb = (unsigned)((nmax + 255) / 256);
+    sort_keys_kernel<<<dim3(nb, ns), 256, 0, c->stream>>>(a);
+    sort_sums_kernel<<<dim3((unsigned)sb, ns), 1024, 0, c->stream>>>(a, sb);
+    sort_offsets_kernel<<<dim3((unsigned)sb, ns), 1024, 0, c->stream>>>(a, sb);
+    scatter_kernel<<<dim3(nb, ns), 256, 0, c->stream>>>(sa);
+    for (int kind = 0; kind < 2; ++kind) {
+        if (!((mask >> kind) & 1)) continue;
+        Species &s = c->sp[kind];
+        std::swap(s.a, s.b);
+        if (s.orig) {
+            std::swap(s.orig, s.orig_b);
+            std::swap(s.dead, s.dead_b);
+            s.perm_fresh = true;
+        }
+        s.sorted = true;
+        s.pushes_since_sort = 0;
+        s.vis_built_for = 0;
+        s.strag_zero = true;
     }
-    sa.is[sa.ni] = s.a.id; sa.id_[sa.ni++] = s.b.id;
-    if (s.orig) {   // adjoint mode: upload index, dead flags, and the permutation for the tape
-        sa.is[sa.ni] = s.orig; sa.id_[sa.ni++] = s.orig_b;
-        sa.bs = s.dead;
-        sa.bd = s.dead_b;
-        sa.perm = s.perm;
+}
+
+// the species of `mask` whose sort is due before their next push
+static int sorts_due(const pic_ctx *c, int mask) {
+    int due = 0;
+    for (int k = 0; k < 2; ++k) {
+        const Species &s = c->sp[k];
+        if (((mask >> k) & 1) && s.n_host > 0 && (!s.sorted || s.pushes_since_sort >= c->sort_interval)) due |= 1 << k;
     }
-    scatter_kernel<<<nb, 256, 0, c->stream>>>(sa);
-    std::swap(s.a, s.b);
-    if (s.orig) {
-        std::swap(s.orig, s.orig_b);
-        std::swap(s.dead, s.dead_b);
-        s.perm_fresh = true;
-    }
-    s.sorted = true;
-    s.pushes_since_sort = 0;
-    if (s.vs) {   // every particle is at home: empty visitor lists
-        cudaMemsetAsync(s.vis_off, 0, (size_t)(c->ntile[0] * c->ntile[1] * c->ntile[2] + 1) * sizeof(unsigned),
-                        c->stream);
-        vis_reset_kernel<<<1, 1, 0, c->stream>>>(s.vs);
-    }
-    s.vis_built_for = 0;
-    prof_end(c);
+    return due;
 }
 
 void launch_sort_due(pic_ctx *c, int mask) {
     if (c->tile <= 0) return;
-    for (int k = 0; k < 2; ++k) {
-        Species &s = c->sp[k];
-        if (!((mask >> k) & 1) || s.n_host <= 0) continue;
-        if (!s.sorted || s.pushes_since_sort >= c->sort_interval) launch_sort(c, k);
+    const int due = sorts_due(c, mask);
+    if (!due) return;
+    prof_begin(c, "sort_particles");
+    if (c->sort_slots == 2) {
+        sort_together(c, due);
+    } else {
+        for (int k = 0; k < 2; ++k)
+            if ((due >> k) & 1) sort_together(c, 1 << k);
     }
+    prof_end(c);
 }
 
 // Before a push: a full sort when due, else this push's visitor lists from
 // what the last push recorded (once per push: pushes_since_sort counts them).
 static void prepare_push(pic_ctx *c, int mask) {
     if (c->tile <= 0) return;
+    launch_sort_due(c, mask);
+    int build = 0;
     for (int k = 0; k < 2; ++k) {
         Species &s = c->sp[k];
         if (!((mask >> k) & 1) || s.n_host <= 0) continue;
-        if (!s.sorted || s.pushes_since_sort >= c->sort_interval) {
-            launch_sort(c, k);
-        } else if (s.vs && s.vis_built_for != s.pushes_since_sort) {
-            prof_begin(c, "visitor_lists");
-            launch_vis_build(c, s);
-            prof_end(c);
-        }
+        if (s.vs && s.vis_built_for != s.pushes_since_sort) build |= 1 << k;
         s.vis_built_for = s.pushes_since_sort;
+    }
+    if (build) {
+        prof_begin(c, "visitor_lists");
+        launch_vis_build(c, build);
+        prof_end(c);
+    }
+    for (int k = 0; k < 2; ++k) {
+        Species &s = c->sp[k];
+        if (!((mask >> k) & 1) || s.n_host <= 0) continue;
+        if (!s.strag_zero) cudaMemsetAsync(c->d_nstrag + k, 0, sizeof(unsigned long long), c->stream);
+        s.strag_zero = false;
     }
 }
 
@@ -507,8 +629,9 @@ __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) tile_push_kernel(Tile
         if (pa[k] > pb[k]) pa[k] = pb[k];
         vvalid[k] = ta.vs[k] && ta.vs[k]->valid_cur;
         if (vvalid[k] && ta.vis_off[k]) {
-            va[k] = ta.vis_off[k][tile];
-            vb[k] = ta.vis_off[k][tile + 1];
+            const uint2 r = ta.vis_off[k][tile];
+            va[k] = r.x;
+            vb[k] = r.y;
         }
         mtot += pb[k] - pa[k] + vb[k] - va[k];
     }
@@ -684,7 +807,9 @@ VisSink vis_sink_of(const pic_ctx *c, const Species &s) {
     VisSink v{};
     if (!s.vs) return v;
     v.raw = s.vraw;
-    v.vs = s.vs;
+    v.nraw = &s.vs->nraw[s.vis_par];
+    v.valid = &s.vs->valid_next[s.vis_par];
+    v.cnt = s.vis_cnt;
     v.cap = s.vcap;
     v.T = c->tile;
     v.nodes = c->node_tiles ? 1 : 0;
@@ -695,7 +820,6 @@ VisSink vis_sink_of(const pic_ctx *c, const Species &s) {
 template <typename real, int P, bool SPIN>
 static void tile_push_t(pic_ctx *c, int mask) {
     const TileArgs<real> ta = make_tile_args<real, P>(c, mask, tile_layout(c));
-    cudaMemsetAsync(c->d_nstrag, 0, 2 * sizeof(unsigned long long), c->stream);
     size_t smem = tile_smem_bytes(c);
     const int ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
     constexpr int NT = tile_threads<real, P>();
@@ -729,9 +853,9 @@ int tile_order_stats(pic_ctx *c, int kind, long long (&out)[4]) {
         if (cudaMemcpy(&v, s.vs, sizeof v, cudaMemcpyDeviceToHost) != cudaSuccess) return PIC_ECUDA;
         if (cudaMemcpy(&n, s.d_count, sizeof n, cudaMemcpyDeviceToHost) != cudaSuccess) return PIC_ECUDA;
         const bool built = s.vis_built_for == s.pushes_since_sort;
-        out[0] = built ? (long long)v.nvis : std::min<long long>((long long)v.nraw, s.vcap);
+        out[0] = built ? (long long)v.nvis : std::min<long long>((long long)v.nraw[s.vis_par], s.vcap);
         out[1] = built ? v.valid_cur
-                       : (v.valid_next && visitor_lists_pay((unsigned long long)out[0], n, visitor_min_fraction(c)));
+                       : (v.valid_next[s.vis_par] && visitor_lists_pay((unsigned long long)out[0], n, visitor_min_fraction(c)));
     }
     if (c->d_nstrag) {
         unsigned long long ns[2] = {0, 0};
@@ -756,9 +880,7 @@ void launch_tile_push(pic_ctx *c, int mask) {
     }
     prof_end(c);
     prof_begin(c, "straggler_push");
-    for (int k = 0; k < 2; ++k)
-        if (((mask >> k) & 1) && c->sp[k].n_host > 0)
-            launch_push_list(c, k, c->sp[k].strag, c->d_nstrag + k, vis_sink_of(c, c->sp[k]));
+    launch_push_stragglers(c, mask);
     prof_end(c);
     for (int k = 0; k < 2; ++k) {
         Species &s = c->sp[k];

@@ -159,8 +159,9 @@ __global__ void __launch_bounds__(NodeTile<real, P>::kThreads, NodeTile<real, P>
         vvalid[k] = ta.vs[k] && ta.vs[k]->valid_cur;
         long long vis = 0;
         if (vvalid[k] && ta.vis_off[k]) {
-            va[k] = ta.vis_off[k][tile];
-            vis = (long long)ta.vis_off[k][tile + 1] - va[k];
+            const uint2 r = ta.vis_off[k][tile];
+            va[k] = r.x;
+            vis = r.y - r.x;
         }
         mtot += home + vis;
         mh[k] = (int)home;
@@ -521,7 +522,6 @@ void node_tile_push(pic_ctx *c, int mask) {
     t.nodes = 1;
     t.nacc = (c->p.deposit_rho && !c->rho_skip) ? 5 : 3;
     const TileArgs<real> ta = make_tile_args<real, P>(c, mask, t);
-    cudaMemsetAsync(c->d_nstrag, 0, 2 * sizeof(unsigned long long), c->stream);
     const int ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
     auto launch = [&](auto kernel) {
         const size_t smem = L::smem(t.nacc);
