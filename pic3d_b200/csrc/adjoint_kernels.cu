@@ -27,6 +27,7 @@
 
 #include "pic_kernels.cuh"
 #include "push_core.cuh"
+#include "tile_common.cuh"
 
 namespace pic {
 
@@ -911,10 +912,13 @@ __global__ void adj_bc_kernel(AdjBcArgs A, real *lex, real *ley, real *lez, real
     const int nc = A.profile_n;
     const double u = ((double)(iy - g.mem) + 0.5) / (double)g.n[1] * (double)(nc - 1);
     const double v = ((double)(iz - g.mem) + 0.5) / (double)g.n[2] * (double)(nc - 1);
-    for (int b = 0; b < nc; ++b) {
+    // the coefficients within two knots (the others' basis is zero)
+    const int b0 = max((int)floor(v) - 1, 0), b1 = min((int)floor(v) + 2, nc - 1);
+    const int c0 = max((int)floor(u) - 1, 0), c1 = min((int)floor(u) + 2, nc - 1);
+    for (int b = b0; b <= b1; ++b) {
         double wv = cubic_bspline(v - b);
         if (wv == 0.0) continue;
-        for (int cidx = 0; cidx < nc; ++cidx) {
+        for (int cidx = c0; cidx <= c1; ++cidx) {
             double wu = cubic_bspline(u - cidx);
             if (wu == 0.0) continue;
             atomicAdd(A.lprof + b * nc + cidx, lsrc * f * wu * wv);
@@ -988,15 +992,46 @@ __global__ void adj_seed_kinetic_kernel(Geom g, CellPack cp, int fp32, long long
 }  // namespace pic
 
 // moves of per-particle arrays between orders (bit copies)
-template <typename T>
-__global__ void scatter_to_kernel(const T *in, const int *to, T *out, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[to[i]] = in[i];
+// Several device arrays of 16-byte aligned addresses copied in one launch
+// (blockIdx.y: the array).  A tape slot has 16 or more of them and is saved
+// before every push: one by one, 1.9 us and a launch each, they took a tenth
+// of a small differentiable run.
+struct CopyList {
+    static constexpr int kMax = 24;
+    const void *src[kMax];
+    void *dst[kMax];
+    unsigned long long bytes[kMax];
+};
+
+__global__ void __launch_bounds__(256) copy_arrays_kernel(const __grid_constant__ CopyList l) {
+    const int a = blockIdx.y;
+    const unsigned long long words = l.bytes[a] / 16, nt = (unsigned long long)gridDim.x * 256;
+    const uint4 *src = (const uint4 *)l.src[a];
+    uint4 *dst = (uint4 *)l.dst[a];
+    for (unsigned long long i = (unsigned long long)blockIdx.x * 256 + threadIdx.x; i < words; i += nt) dst[i] = src[i];
+    const unsigned tail = (unsigned)(l.bytes[a] & 15);
+    if (blockIdx.x == 0 && threadIdx.x < tail)
+        ((unsigned char *)dst)[words * 16 + threadIdx.x] = ((const unsigned char *)src)[words * 16 + threadIdx.x];
 }
-template <typename T>
-__global__ void gather_from_kernel(const T *in, const int *from, T *out, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in[from[i]];
+
+// The same permutation of several per-particle arrays in one launch:
+// out[map[i]] = in[i], or (GATHER) out[i] = in[map[i]].
+struct PermuteList {
+    const unsigned long long *ds[8];
+    unsigned long long *dd[8];
+    int nd;
+    const unsigned *fs[8];
+    unsigned *fd[8];
+    int nf;
+};
+
+template <bool GATHER>
+__global__ void __launch_bounds__(256) permute_kernel(const __grid_constant__ PermuteList l, const int *map, long long n) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const long long j = map[i], from = GATHER ? j : i, to = GATHER ? i : j;
+    pic::move_words(l.ds, l.dd, l.nd, from, to);
+    pic::move_words(l.fs, l.fd, l.nf, from, to);
 }
 
 // ===========================================================================
@@ -1035,8 +1070,9 @@ struct AdjState {
     int *lam_orig[2] = {};
     bool lam_valid = false;
     unsigned *toffs[2] = {};   // tiled contexts: tile boundaries extracted for the tape
-    void *tmp = nullptr;
-    size_t tmp_bytes = 0;
+    // second set of the per-particle arrays: where a permutation goes
+    void *lpart_b[2][6] = {};
+    double *lw_b[2] = {};
 };
 
 static std::vector<std::pair<pic_ctx *, AdjState *>> g_adj;
@@ -1090,6 +1126,28 @@ static void checkpoint_parts(pic_ctx *c, std::vector<std::pair<void *, size_t>> 
     for (int f = 0; f < 5; ++f) v.push_back({c->ring[f], (size_t)c->g.rsz * rsize(c)});
 }
 
+// between the parts and their places in the blob, as many arrays per launch
+// as a list holds
+static void copy_parts(pic_ctx *c, const Blob &b, const std::vector<std::pair<void *, size_t>> &parts, bool save) {
+    size_t off = 0;
+    for (size_t i = 0; i < parts.size();) {
+        CopyList l{};
+        int m = 0;
+        size_t most = 0;
+        for (; i < parts.size() && m < CopyList::kMax; ++i, ++m) {
+            void *in_blob = (char *)b.buf + off;
+            l.src[m] = save ? parts[i].first : in_blob;
+            l.dst[m] = save ? in_blob : parts[i].first;
+            l.bytes[m] = parts[i].second;
+            most = std::max(most, parts[i].second);
+            off += (parts[i].second + 255) & ~(size_t)255;
+        }
+        // four words per thread, at most 4 blocks per SM for one array
+        const unsigned grid = (unsigned)std::min<size_t>(most / 16 / 1024 + 1, 148 * 4);
+        copy_arrays_kernel<<<dim3(grid, (unsigned)m), 256, 0, c->stream>>>(l);
+    }
+}
+
 static int blob_save(pic_ctx *c, Blob &b, const std::vector<std::pair<void *, size_t>> &parts) {
     size_t total = 0;
     for (auto &p : parts) total += (p.second + 255) & ~(size_t)255;
@@ -1104,11 +1162,7 @@ static int blob_save(pic_ctx *c, Blob &b, const std::vector<std::pair<void *, si
         b.bytes = total;
     }
     b.parts = parts;
-    size_t off = 0;
-    for (auto &p : parts) {
-        cudaMemcpyAsync((char *)b.buf + off, p.first, p.second, cudaMemcpyDeviceToDevice, c->stream);
-        off += (p.second + 255) & ~(size_t)255;
-    }
+    copy_parts(c, b, parts, true);
     b.step = c->step;
     for (int k = 0; k < 2; ++k) {
         b.cur[k] = c->sp[k].cur;
@@ -1177,7 +1231,9 @@ static int ensure_adj_arrays(pic_ctx *c, AdjState *A) {
     };
     bool ok = true;
     for (int f = 0; f < 6; ++f) ok = ok && alloc(&A->lf[f], (size_t)c->g.fsz * rs);
-    for (int f = 0; f < 3; ++f) ok = ok && alloc(&A->lj[f], (size_t)c->g.rsz * rs);
+    // the three J adjoints in one block: cleared by one memset
+    ok = ok && alloc(&A->lj[0], 3 * (size_t)c->g.rsz * rs);
+    for (int f = 1; f < 3 && ok; ++f) A->lj[f] = (char *)A->lj[0] + (size_t)f * c->g.rsz * rs;
     for (int k = 0; k < 2; ++k) {
         size_t n = (size_t)std::max<int64_t>(c->sp[k].cap, 1);
         for (int q = 0; q < 6; ++q) ok = ok && alloc(&A->lpart[k][q], n * rs);
@@ -1186,14 +1242,12 @@ static int ensure_adj_arrays(pic_ctx *c, AdjState *A) {
     ok = ok && alloc((void **)&A->loss, sizeof(double));
     if (c->sp[0].orig || c->sp[1].orig) {
         size_t n = (size_t)std::max<int64_t>(std::max(c->sp[0].cap, c->sp[1].cap), 1);
-        for (int k = 0; k < 2; ++k) ok = ok && alloc((void **)&A->lam_orig[k], n * sizeof(int));
-        if (A->tmp_bytes < n * sizeof(double)) {
-            if (A->tmp) cudaFree(A->tmp);
-            A->tmp = nullptr;
-            A->tmp_bytes = 0;
+        for (int k = 0; k < 2; ++k) {
+            ok = ok && alloc((void **)&A->lam_orig[k], n * sizeof(int));
+            size_t nk = (size_t)std::max<int64_t>(c->sp[k].cap, 1);
+            for (int q = 0; q < 6; ++q) ok = ok && alloc(&A->lpart_b[k][q], nk * rs);
+            ok = ok && alloc((void **)&A->lw_b[k], nk * sizeof(double));
         }
-        ok = ok && alloc(&A->tmp, n * sizeof(double));
-        if (ok) A->tmp_bytes = n * sizeof(double);
     }
     int np = std::max(c->profile_n * c->profile_n, 1);
     if (A->nprof != np && A->lprof) {
@@ -1209,41 +1263,47 @@ static int ensure_adj_arrays(pic_ctx *c, AdjState *A) {
     return PIC_OK;
 }
 
-// the per-particle arrays a sort moves that the reverse sweep reads:
-// position and momentum adjoints, weight adjoint, weights, upload index
-static int moved_arrays(pic_ctx *c, AdjState *A, int k, void **arr, size_t *es) {
-    int m = 0;
-    for (int q = 0; q < 6; ++q) { arr[m] = A->lpart[k][q]; es[m++] = rsize(c); }
-    arr[m] = A->lw[k]; es[m++] = sizeof(double);
-    arr[m] = c->sp[k].a.w; es[m++] = rsize(c);
-    arr[m] = c->sp[k].orig; es[m++] = sizeof(int);
-    return m;
+// The per-particle arrays a sort moves that the reverse sweep reads: the
+// adjoints (position, momentum, weight) and, if `all`, weights and upload
+// index; between the first and the second set of arrays.
+static PermuteList moved_arrays(pic_ctx *c, AdjState *A, int k, bool all, bool back) {
+    PermuteList l{};
+    auto add = [&](void *a, void *b, size_t es) {
+        if (back) std::swap(a, b);
+        if (es == 8) {
+            l.ds[l.nd] = (const unsigned long long *)a;
+            l.dd[l.nd++] = (unsigned long long *)b;
+        } else {
+            l.fs[l.nf] = (const unsigned *)a;
+            l.fd[l.nf++] = (unsigned *)b;
+        }
+    };
+    Species &s = c->sp[k];
+    for (int q = 0; q < 6; ++q) add(A->lpart[k][q], A->lpart_b[k][q], rsize(c));
+    add(A->lw[k], A->lw_b[k], sizeof(double));
+    if (all) {
+        add(s.a.w, s.b.w, rsize(c));
+        add(s.orig, s.orig_b, sizeof(int));
+    }
+    return l;
 }
 
-static void scatter_to(pic_ctx *c, const void *in, const int *to, void *out, size_t es, long long n) {
+static void permute(pic_ctx *c, const PermuteList &l, const int *map, long long n, bool gather) {
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (es == 8) scatter_to_kernel<unsigned long long><<<blocks, 256, 0, c->stream>>>(
-        (const unsigned long long *)in, to, (unsigned long long *)out, n);
-    else scatter_to_kernel<unsigned><<<blocks, 256, 0, c->stream>>>((const unsigned *)in, to, (unsigned *)out, n);
-}
-
-static void gather_from(pic_ctx *c, const void *in, const int *from, void *out, size_t es, long long n) {
-    const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (es == 8) gather_from_kernel<unsigned long long><<<blocks, 256, 0, c->stream>>>(
-        (const unsigned long long *)in, from, (unsigned long long *)out, n);
-    else gather_from_kernel<unsigned><<<blocks, 256, 0, c->stream>>>((const unsigned *)in, from, (unsigned *)out, n);
+    if (gather) permute_kernel<true><<<blocks, 256, 0, c->stream>>>(l, map, n);
+    else permute_kernel<false><<<blocks, 256, 0, c->stream>>>(l, map, n);
 }
 
 // undo one recorded sort of species k (perm[new] = old): every moved array
-// goes back to the order before that sort
+// goes back to the order before that sort, into the other set, which becomes
+// the first
 static void unsort_species(pic_ctx *c, AdjState *A, int k, const int *perm, long long n) {
-    void *arr[9];
-    size_t es[9];
-    const int m = moved_arrays(c, A, k, arr, es);
-    for (int q = 0; q < m; ++q) {
-        cudaMemcpyAsync(A->tmp, arr[q], (size_t)n * es[q], cudaMemcpyDeviceToDevice, c->stream);
-        scatter_to(c, A->tmp, perm, arr[q], es[q], n);
-    }
+    permute(c, moved_arrays(c, A, k, true, false), perm, n, false);
+    Species &s = c->sp[k];
+    for (int q = 0; q < 6; ++q) std::swap(A->lpart[k][q], A->lpart_b[k][q]);
+    std::swap(A->lw[k], A->lw_b[k]);
+    std::swap(s.a.w, s.b.w);
+    std::swap(s.orig, s.orig_b);
 }
 
 // the adjoints are held in the order given by lam_orig (upload indices);
@@ -1256,13 +1316,8 @@ static void remap_adjoints(pic_ctx *c, AdjState *A) {
         Species &s = c->sp[k];
         const long long n = s.n_host;
         if (!s.orig || n == 0) continue;
-        void *arr[9];
-        size_t es[9];
-        const int m = moved_arrays(c, A, k, arr, es) - 2;   // the adjoints only (weights, orig are current)
-        for (int q = 0; q < m; ++q) {
-            scatter_to(c, arr[q], A->lam_orig[k], A->tmp, es[q], n);
-            gather_from(c, A->tmp, s.orig, arr[q], es[q], n);
-        }
+        permute(c, moved_arrays(c, A, k, false, false), A->lam_orig[k], n, false);
+        permute(c, moved_arrays(c, A, k, false, true), s.orig, n, true);
     }
 }
 
@@ -1427,7 +1482,7 @@ static int adj_backward_t(pic_ctx *c, AdjState *A, int nsteps) {
             if (b.perm_part[k] >= 0) unsort_species(c, A, k, (const int *)blob_part(b, b.perm_part[k]), b.count[k]);
         // clear_currents: J before the clear does not reach the deposit
         prof_begin(c, "adjoint_clear");
-        for (int f = 0; f < 3; ++f) cudaMemsetAsync(A->lj[f], 0, (size_t)c->g.rsz * rsize(c), c->stream);
+        cudaMemsetAsync(A->lj[0], 0, 3 * (size_t)c->g.rsz * rsize(c), c->stream);
         prof_end(c);
         if (loop) {
             // first half (field.cpp:56-86): E then B forward
@@ -1477,11 +1532,7 @@ int pic_checkpoint_restore(pic_ctx *c, int slot) {
         c->err = "checkpoint layout differs from the context's";
         return PIC_EINVAL;
     }
-    size_t off = 0;
-    for (size_t i = 0; i < parts.size(); ++i) {
-        cudaMemcpyAsync(parts[i].first, (char *)b.buf + off, parts[i].second, cudaMemcpyDeviceToDevice, c->stream);
-        off += (parts[i].second + 255) & ~(size_t)255;
-    }
+    copy_parts(c, b, parts, false);
     for (int k = 0; k < 2; ++k) {
         c->sp[k].sorted = false;   // the next push sorts (and the tape records that permutation)
         c->sp[k].perm_fresh = false;
@@ -1532,7 +1583,7 @@ int pic_adjoint_seed_kinetic(pic_ctx *c, int kind, double xlo, double xhi, doubl
     if (r) return r;
     const size_t rs = rsize(c);
     for (int f = 0; f < 6; ++f) cudaMemsetAsync(A->lf[f], 0, (size_t)c->g.fsz * rs, c->stream);
-    for (int f = 0; f < 3; ++f) cudaMemsetAsync(A->lj[f], 0, (size_t)c->g.rsz * rs, c->stream);
+    cudaMemsetAsync(A->lj[0], 0, 3 * (size_t)c->g.rsz * rs, c->stream);
     for (int k = 0; k < 2; ++k) {
         size_t n = (size_t)std::max<int64_t>(c->sp[k].cap, 1);
         for (int q = 0; q < 6; ++q) cudaMemsetAsync(A->lpart[k][q], 0, n * rs, c->stream);
@@ -1584,8 +1635,12 @@ int pic_adjoint_weight_grad(pic_ctx *c, int kind, double *out, int64_t n) {
     const double *src = A->lw[kind];
     Species &s = c->sp[kind];
     if (s.orig && n > 0 && s.n_host > 0) {   // sorted context: back to upload order
-        scatter_to(c, A->lw[kind], s.orig, A->tmp, sizeof(double), s.n_host);
-        src = (const double *)A->tmp;
+        PermuteList l{};
+        l.ds[0] = (const unsigned long long *)A->lw[kind];
+        l.dd[0] = (unsigned long long *)A->lw_b[kind];
+        l.nd = 1;
+        permute(c, l, s.orig, s.n_host, false);
+        src = A->lw_b[kind];
     }
     cudaMemcpyAsync(out, src, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
     return cudaStreamSynchronize(c->stream) == cudaSuccess ? PIC_OK : PIC_ECUDA;
@@ -1610,14 +1665,15 @@ int pic_adjoint_release(pic_ctx *c) {
         for (auto &b : A->tape)
             if (b.buf) cudaFree(b.buf);
         for (void *p : A->lf) if (p) cudaFree(p);
-        for (void *p : A->lj) if (p) cudaFree(p);
+        if (A->lj[0]) cudaFree(A->lj[0]);
         for (auto &sp : A->lpart) for (void *p : sp) if (p) cudaFree(p);
         for (double *p : A->lw) if (p) cudaFree(p);
         if (A->lprof) cudaFree(A->lprof);
         if (A->loss) cudaFree(A->loss);
         for (int *p : A->lam_orig) if (p) cudaFree(p);
         for (unsigned *p : A->toffs) if (p) cudaFree(p);
-        if (A->tmp) cudaFree(A->tmp);
+        for (auto &sp : A->lpart_b) for (void *p : sp) if (p) cudaFree(p);
+        for (double *p : A->lw_b) if (p) cudaFree(p);
         delete A;
         g_adj.erase(g_adj.begin() + (long)i);
         return PIC_OK;

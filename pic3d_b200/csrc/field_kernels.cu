@@ -395,10 +395,13 @@ __device__ double gpulse(const LaserArgs &L, const Geom &g, double time, double 
         double u = ((double)(iy - g.mem) + 0.5) / (double)g.n[1] * (double)(nc - 1);
         double v = ((double)(iz - g.mem) + 0.5) / (double)g.n[2] * (double)(nc - 1);
         amp = 0.0;
-        for (int b = 0; b < nc; ++b) {
+        // the coefficients within two knots (the others' basis is zero)
+        const int b0 = max((int)floor(v) - 1, 0), b1 = min((int)floor(v) + 2, nc - 1);
+        const int c0 = max((int)floor(u) - 1, 0), c1 = min((int)floor(u) + 2, nc - 1);
+        for (int b = b0; b <= b1; ++b) {
             double wv = cubic_bspline(v - b);
             if (wv == 0.0) continue;
-            for (int c = 0; c < nc; ++c) {
+            for (int c = c0; c <= c1; ++c) {
                 double wu = cubic_bspline(u - c);
                 if (wu == 0.0) continue;
                 amp += L.coef[b * nc + c] * wu * wv;

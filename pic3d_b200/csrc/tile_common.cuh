@@ -44,6 +44,23 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src, int src_byt
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+// moves element i of n arrays to dst, the loads of eight arrays before their
+// stores (the compiler must assume that a store changes the next source)
+template <typename T, int N>
+__device__ __forceinline__ void move_words(const T *const (&src)[N], T *const (&to)[N], int n, long long i, long long dst) {
+#pragma unroll
+    for (int k0 = 0; k0 < N; k0 += 8) {
+        if (k0 >= n) break;
+        T v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < N && k0 + k < n) v[k] = src[k0 + k][i];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k0 + k < N && k0 + k < n) to[k0 + k][dst] = v[k];
+    }
+}
+
 // word offset (from the accumulators) of the particle input buffers: after
 // the five accumulators, rounded up to 16 bytes
 __host__ __device__ constexpr int particle_buffer_offset(int acc_words) { return (acc_words + 3) & ~3; }

@@ -247,23 +247,6 @@ struct ScatterArgs {
     } s[2];
 };
 
-// moves element i of n arrays to dst, the loads of eight arrays before their
-// stores (the compiler must assume that a store changes the next source)
-template <typename T, int N>
-__device__ __forceinline__ void move_words(const T *const (&src)[N], T *const (&to)[N], int n, long long i, unsigned dst) {
-#pragma unroll
-    for (int k0 = 0; k0 < N; k0 += 8) {
-        if (k0 >= n) break;
-        T v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k0 + k < N && k0 + k < n) v[k] = src[k0 + k][i];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k0 + k < N && k0 + k < n) to[k0 + k][dst] = v[k];
-    }
-}
-
 __global__ void __launch_bounds__(256) scatter_kernel(const __grid_constant__ ScatterArgs sa) {
     const ScatterArgs::One &a = sa.s[blockIdx.y];
     long long n = *a.count;
@@ -285,8 +268,8 @@ __global__ void __launch_bounds__(256) scatter_kernel(const __grid_constant__ Sc
         atomicOr(sa.status, ST_OVERFLOW);
         return;
     }
-    move_words(a.ds, a.dd, a.nd, i, dst);
-    move_words(a.fs, a.fd, a.nf, i, dst);
+    move_words(a.ds, a.dd, a.nd, i, (long long)dst);
+    move_words(a.fs, a.fd, a.nf, i, (long long)dst);
     if (a.bs) a.bd[dst] = a.bs[i];
     if (a.perm) a.perm[dst] = (int)i;
 }
