@@ -88,6 +88,10 @@ bool node_tiles_for(int tile, bool adjoint, int order);   // whether a context u
 size_t node_tile_smem_bytes(const pic_ctx *c);
 void launch_node_tile_kernel(pic_ctx *c, int mask, bool spin);
 
+// tile_node_kernels.cu: the same at 2nd order
+size_t node_sum_smem_bytes(const pic_ctx *c);
+void launch_node_sum_kernel(pic_ctx *c, int mask, bool spin);
+
 // adjoint_kernels.cu
 void adjoint_record_hook(pic_ctx *c);
 

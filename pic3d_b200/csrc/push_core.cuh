@@ -356,10 +356,11 @@ __device__ __forceinline__ void mid_loop(int len, const real (&s0)[P + 1], const
 // Esirkepov deposit (src/particle.cpp:427-500) and rho (:503-514) from the
 // three axes' factors.  The last point of each running sum (the sum of all
 // ds, zero up to rounding) is not added.  `moved`: the particle changed
-// position (one at rest adds no current, only rho).
+// position (one at rest adds no current, only rho).  parts: which of jx, jy,
+// jz, rho to add.
 template <typename real, int P, class Acc>
 __device__ __forceinline__ void deposit(const Acc &acc, const real (&dxdt)[3], const Axis1D<real, P> (&ax)[3],
-                                        bool moved, real qw) {
+                                        bool moved, real qw, unsigned parts = 15u) {
     constexpr int H = P / 2;
     const int base[3] = {ax[0].base, ax[1].base, ax[2].base};
     const int len[3] = {ax[0].len, ax[1].len, ax[2].len};
@@ -380,7 +381,7 @@ __device__ __forceinline__ void deposit(const Acc &acc, const real (&dxdt)[3], c
     if (moved) {
         // Jx: running sum of ds along x times the yz weight
 #pragma unroll 1
-        for (int k = 0; k < len[2]; ++k) {
+        for (int k = 0; (parts & 1u) && k < len[2]; ++k) {
             const real sz0 = pick(s0z, k), szd = pick(dsz, k);
             mid_loop<kRollMid, P>(len[1], s0y, dsy, [&](int j, real sy0, real syd) {
                 const real wyz = sy0 * sz0 + half * syd * sz0 + half * sy0 * szd + third * syd * szd;
@@ -397,7 +398,7 @@ __device__ __forceinline__ void deposit(const Acc &acc, const real (&dxdt)[3], c
         }
         // Jy
 #pragma unroll 1
-        for (int k = 0; k < len[2]; ++k) {
+        for (int k = 0; (parts & 2u) && k < len[2]; ++k) {
             const real sz0 = pick(s0z, k), szd = pick(dsz, k);
             mid_loop<kRollMid, P>(len[0], s0x, dsx, [&](int i, real sx0, real sxd) {
                 const real wxz = sx0 * sz0 + half * sxd * sz0 + half * sx0 * szd + third * sxd * szd;
@@ -414,7 +415,7 @@ __device__ __forceinline__ void deposit(const Acc &acc, const real (&dxdt)[3], c
         }
         // Jz
 #pragma unroll 1
-        for (int j = 0; j < len[1]; ++j) {
+        for (int j = 0; (parts & 4u) && j < len[1]; ++j) {
             const real sy0 = pick(s0y, j), syd = pick(dsy, j);
             mid_loop<kRollMid, P>(len[0], s0x, dsx, [&](int i, real sx0, real sxd) {
                 const real wxy = sx0 * sy0 + half * sxd * sy0 + half * sx0 * syd + third * sxd * syd;
@@ -430,7 +431,7 @@ __device__ __forceinline__ void deposit(const Acc &acc, const real (&dxdt)[3], c
             });
         }
     }
-    if (acc.has_rho()) {
+    if (acc.has_rho() && (parts & 8u)) {
         const real qwr = qw * acc.coef(3);
         const int rb = (ax[2].i2 - H) * rxy + (ax[1].i2 - H) * rx + (ax[0].i2 - H) + acc.o;
 #pragma unroll 1
@@ -734,6 +735,39 @@ __device__ __forceinline__ bool push_move(const PushArgs<real> &a, long long p, 
         }
     }
     return true;
+}
+
+// The deposit of particle p after its push, from its stored old and new
+// position (and, FP32, the new momentum, which gives its move in cells).
+template <typename real, int P, class Acc>
+__device__ __forceinline__ void deposit_stored(const Acc &acc, const PushArgs<real> &a, int p, unsigned parts) {
+    const Geom &g = a.g;
+    Axis1D<real, P> ax[3];
+    if constexpr (sizeof(real) == 8) {
+        const double *x0[3] = {a.x0, a.y0, a.z0}, *x1[3] = {a.x1, a.y1, a.z1};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double o = __ldcg(x0[d] + p) - (double)(1 - g.mem), n = __ldcg(x1[d] + p) - (double)(1 - g.mem);
+            const int i1 = (int)(o + 0.5), i2 = (int)(n + 0.5);
+            axis_from_offsets<real, P>(i1, o - (double)i1, i2, n - (double)i2, ax[d]);
+        }
+    } else {
+        const float *o0[3] = {a.ox0, a.oy0, a.oz0}, *o1[3] = {a.ox1, a.oy1, a.oz1};
+        const float pn[3] = {__ldcg(a.px + p), __ldcg(a.py + p), __ldcg(a.pz + p)};
+        const float ig = inv_sqrt(1.0f + (pn[0] * pn[0] + pn[1] * pn[1] + pn[2] * pn[2]));
+        int c0[3], c1[3];
+        a.cp.unpack(__ldcg(a.c0 + p), c0[0], c0[1], c0[2]);
+        a.cp.unpack(__ldcg(a.c1 + p), c1[0], c1[1], c1[2]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float f0 = __ldcg(o0[d] + p), f1 = __ldcg(o1[d] + p);
+            int step = c1[d] - c0[d];   // -1, 0 or 1 before the periodic wrap
+            if (g.per[d]) step = step > 1 ? step - g.n[d] : (step < -1 ? step + g.n[d] : step);
+            const int b = c0[d] + g.mem - 1, i1 = b + (f0 >= 0.5f ? 1 : 0), i2 = b + step + (f1 >= 0.5f ? 1 : 0);
+            axis_from_move<P>(i1, f0 >= 0.5f ? f0 - 1.0f : f0, pn[d] * ig * a.dt_d[d], i2, ax[d]);
+        }
+    }
+    deposit<real, P>(acc, a.d_dt, ax, true, a.charge * __ldcg(a.w + p), parts);
 }
 
 // push_move, then the particle's deposit into acc.  The new state is stored

@@ -534,20 +534,23 @@ void node_tile_push(pic_ctx *c, int mask) {
 
 }  // namespace
 
-// Tiles of nodes with the matrix deposit: 4th order at the default tile
-// edge.  Measured per launch on 128 x 64 x 64 cells, 8 + 8 particles per cell
-// (tiles of cells with a scatter per particle first): FP64 7.08 -> 4.07 ms,
-// FP32 3.72 -> 2.42 ms.  At 2nd order a particle's 54 points cost less to
-// scatter (FP32 1.01 ms) than the factors of its matrix products cost to
-// make (1.23 ms), so it keeps the tiles of cells of tile_kernels.cu, as do
-// other edges and adjoint contexts (whose reverse sweep shares the tiles).
-bool node_tiles_for(int tile, bool adjoint, int order) { return tile == 4 && !adjoint && order == 4; }
+// Tiles of nodes: both orders at the default tile edge.  The matrix deposit
+// here is for 4th order; measured per launch on 128 x 64 x 64 cells, 8 + 8
+// particles per cell (tiles of cells with a scatter per particle first): FP64
+// 7.08 -> 4.07 ms, FP32 3.72 -> 2.42 ms.  At 2nd order the factors of its
+// products cost more to make (FP32 1.23 ms) than a particle's 54 points to
+// scatter (1.01 ms): tile_node_kernels.cu sums them per node instead.  Other
+// edges and adjoint contexts (whose reverse sweep shares the tiles) keep the
+// tiles of cells of tile_kernels.cu.
+bool node_tiles_for(int tile, bool adjoint, int order) { return tile == 4 && !adjoint && (order == 2 || order == 4); }
 
 size_t node_tile_smem_bytes(const pic_ctx *c) {
+    if (c->order == 2) return node_sum_smem_bytes(c);
     return c->fp32 ? NodeTile<float, 5>::smem(5) : NodeTile<double, 5>::smem(5);
 }
 
 void launch_node_tile_kernel(pic_ctx *c, int mask, bool spin) {
+    if (c->order == 2) return launch_node_sum_kernel(c, mask, spin);
     if (c->fp32) spin ? node_tile_push<float, 5, true>(c, mask) : node_tile_push<float, 5, false>(c, mask);
     else spin ? node_tile_push<double, 5, true>(c, mask) : node_tile_push<double, 5, false>(c, mask);
 }
