@@ -15,11 +15,11 @@
 //   * BC transpose: one thread per face row; adds into neighbours with
 //     atomics and accumulates d objective / d(profile coefficient).
 //   * push adjoint: one thread per particle; recomputes the gather with
-//     shape-derivative weights, takes the Boris Jacobian by forward-mode
-//     dual numbers (three passes of three tangents), contracts the current
-//     adjoint with the Esirkepov factors to get the derivatives of the
-//     deposit with respect to the old and new positions and the weight,
-//     and scatters the gathered-field adjoints back to the grid.
+//     shape-derivative weights, contracts the current adjoint with the
+//     Esirkepov factors to get the derivatives of the deposit with respect
+//     to the old and new positions and the weight, applies the transpose of
+//     the Boris rotation and scatters the gathered-field adjoints back to
+//     the grid.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -32,99 +32,85 @@
 namespace pic {
 
 // ---------------------------------------------------------------------------
-// forward-mode dual numbers with N tangents
-
-template <typename T, int N>
-struct Dual {
-    T v;
-    T d[N];
+// Boris rotation and move (particle.cpp:271-315) of one particle, and its
+// transpose.  (The Jacobian by forward-mode dual numbers, three passes of three
+// tangents, took about 2000 instructions per particle; the transpose takes
+// some 130 beside the values.)
+template <typename T>
+struct Boris {
+    T e[3], b[3], p1[3], t[3], s[3], p2[3], pn[3];
+    T ig1, f, ig;   // 1 / gamma of p1, 2 / (1 + t^2), 1 / gamma of pn
 };
 
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> dconst(T v) {
-    Dual<T, N> r;
-    r.v = v;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = T(0);
-    return r;
-}
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> operator+(const Dual<T, N> &a, const Dual<T, N> &b) {
-    Dual<T, N> r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] + b.d[i];
-    return r;
-}
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> operator-(const Dual<T, N> &a, const Dual<T, N> &b) {
-    Dual<T, N> r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] - b.d[i];
-    return r;
-}
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> operator*(const Dual<T, N> &a, const Dual<T, N> &b) {
-    Dual<T, N> r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * b.v + a.v * b.d[i];
-    return r;
-}
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> operator*(const Dual<T, N> &a, T s) {
-    Dual<T, N> r;
-    r.v = a.v * s;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * s;
-    return r;
-}
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> operator/(const Dual<T, N> &a, const Dual<T, N> &b) {
-    Dual<T, N> r;
-    T inv = T(1) / b.v;
-    r.v = a.v * inv;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = (a.d[i] - r.v * b.d[i]) * inv;
-    return r;
-}
-template <typename T, int N>
-__device__ __forceinline__ Dual<T, N> dsqrt(const Dual<T, N> &a) {
-    Dual<T, N> r;
-    r.v = sqrt(a.v);
-    T h = T(0.5) / r.v;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r.d[i] = a.d[i] * h;
-    return r;
+template <typename T>
+__device__ __forceinline__ void cross_add(const T (&a)[3], const T (&b)[3], T (&r)[3]) {
+    r[0] += a[1] * b[2] - a[2] * b[1];
+    r[1] += a[2] * b[0] - a[0] * b[2];
+    r[2] += a[0] * b[1] - a[1] * b[0];
 }
 
-// Boris rotation and move (particle.cpp:271-315) on duals; inputs p, e, b
-// (fields unscaled), outputs p' and the displacement in cells
-template <typename T, int N>
-__device__ __forceinline__ void boris_dual(const Dual<T, N> (&p)[3], const Dual<T, N> (&e)[3],
-                                           const Dual<T, N> (&b)[3], T qm, const T (&dtd)[3], Dual<T, N> (&pn)[3],
-                                           Dual<T, N> (&disp)[3]) {
-    Dual<T, N> ep[3], bp[3], p1[3];
+// inputs p, fields e, b (unscaled)
+template <typename T>
+__device__ __forceinline__ void boris_values(const T (&p)[3], const T *e, const T *b, T qm, Boris<T> &v) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        ep[d] = e[d] * qm;
-        bp[d] = b[d] * qm;
-        p1[d] = p[d] + ep[d];
+        v.e[d] = e[d] * qm;
+        v.b[d] = b[d] * qm;
+        v.p1[d] = p[d] + v.e[d];
     }
-    Dual<T, N> one = dconst<T, N>(T(1));
-    Dual<T, N> gm1 = dsqrt(one + (p1[0] * p1[0] + p1[1] * p1[1] + p1[2] * p1[2]));
-    Dual<T, N> t[3] = {bp[0] / gm1, bp[1] / gm1, bp[2] / gm1};
-    Dual<T, N> tt = dconst<T, N>(T(2)) / (one + t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
-    Dual<T, N> s[3] = {t[0] * tt, t[1] * tt, t[2] * tt};
-    Dual<T, N> p2[3] = {p1[0] + (p1[1] * t[2] - p1[2] * t[1]), p1[1] + (p1[2] * t[0] - p1[0] * t[2]),
-                        p1[2] + (p1[0] * t[1] - p1[1] * t[0])};
-    pn[0] = p1[0] + (p2[1] * s[2] - p2[2] * s[1]) + ep[0];
-    pn[1] = p1[1] + (p2[2] * s[0] - p2[0] * s[2]) + ep[1];
-    pn[2] = p1[2] + (p2[0] * s[1] - p2[1] * s[0]) + ep[2];
-    Dual<T, N> gam = dsqrt(one + (pn[0] * pn[0] + pn[1] * pn[1] + pn[2] * pn[2]));
+    v.ig1 = T(1) / sqrt(T(1) + (v.p1[0] * v.p1[0] + v.p1[1] * v.p1[1] + v.p1[2] * v.p1[2]));
 #pragma unroll
-    for (int d = 0; d < 3; ++d) disp[d] = (pn[d] / gam) * dtd[d];
+    for (int d = 0; d < 3; ++d) v.t[d] = v.b[d] * v.ig1;
+    v.f = T(2) / (T(1) + v.t[0] * v.t[0] + v.t[1] * v.t[1] + v.t[2] * v.t[2]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        v.s[d] = v.t[d] * v.f;
+        v.p2[d] = v.p1[d];
+        v.pn[d] = v.p1[d] + v.e[d];
+    }
+    cross_add(v.p1, v.t, v.p2);
+    cross_add(v.p2, v.s, v.pn);
+    v.ig = T(1) / sqrt(T(1) + (v.pn[0] * v.pn[0] + v.pn[1] * v.pn[1] + v.pn[2] * v.pn[2]));
+}
+
+// lin = J^T (lp, lx), J = d(p', displacement in cells) / d(p, e, b); the
+// displacement is pn ig dtd.  Uses grad_a a x b . l = b x l and
+// grad_b a x b . l = l x a.
+template <typename T>
+__device__ __forceinline__ void boris_transpose(const Boris<T> &v, T qm, const T (&dtd)[3], const T (&lp)[3],
+                                                const T (&lx)[3], T (&lin)[9]) {
+    T l[3], li = 0;   // adjoints of pn and ig
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const T q = lx[d] * dtd[d];
+        l[d] = lp[d] + q * v.ig;
+        li += q * v.pn[d];
+    }
+    li *= v.ig * v.ig * v.ig;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) l[d] -= li * v.pn[d];
+    // pn = p1 + p2 x s + e
+    T l1[3] = {l[0], l[1], l[2]}, l2[3] = {0, 0, 0}, ls[3] = {0, 0, 0}, lt[3] = {0, 0, 0};
+    cross_add(v.s, l, l2);
+    cross_add(l, v.p2, ls);
+    // p2 = p1 + p1 x t
+#pragma unroll
+    for (int d = 0; d < 3; ++d) l1[d] += l2[d];
+    cross_add(v.t, l2, l1);
+    cross_add(l2, v.p1, lt);
+    // s = t f, f = 2 / (1 + t^2)
+    const T k = v.f * v.f * (ls[0] * v.t[0] + ls[1] * v.t[1] + ls[2] * v.t[2]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) lt[d] += v.f * ls[d] - k * v.t[d];
+    // t = b ig1
+    const T k1 = v.ig1 * v.ig1 * v.ig1 * (lt[0] * v.b[0] + lt[1] * v.b[1] + lt[2] * v.b[2]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        l1[d] -= k1 * v.p1[d];
+        lin[d] = l1[d];
+        lin[3 + d] = qm * (l[d] + l1[d]);
+        lin[6 + d] = qm * v.ig1 * lt[d];
+    }
 }
 
 // derivatives of the shape weights with respect to the position
@@ -217,36 +203,35 @@ __device__ __forceinline__ void span_pair(int i1, const T (&a0)[P], int i2, cons
     }
 }
 
-// Adjoint of one Esirkepov component.  Axis `c` carries the running sum of
-// ds = s1 - s0, axes `u` and `v` the weight
-// W = 1/3 s0u s0v + 1/6 s1u s0v + 1/6 s0u s1v + 1/3 s1u s1v.
-// Returns G1 = sum(lam * J) / w and adds dG1/ds0, dG1/ds1 into g0, g1.
+// Adjoint of one Esirkepov component in the factors s = (s0 + s1)/2 and
+// d = (s1 - s0)/sqrt(12) of each axis.  Axis `c` carries the running sum of
+// ds = sqrt(12) d, axes `u` and `v` the weight W = s_u s_v + d_u d_v (two
+// products where the four of the old and new shapes took six).  Returns
+// G1 = sum(lam * J) / w and adds dG1/ds, dG1/dd into gs, gd.
 template <int P, bool LDG, typename LT>
 __device__ __forceinline__ double esirkepov_adj(const LT *lam, int sc, int su, int sv, int lc, int lu, int lv,
-                                                double coef, const double (&s0c)[P + 1], const double (&s1c)[P + 1],
-                                                const double (&s0u)[P + 1], const double (&s1u)[P + 1],
-                                                const double (&s0v)[P + 1], const double (&s1v)[P + 1],
-                                                double (&g0c)[P + 1], double (&g1c)[P + 1], double (&g0u)[P + 1],
-                                                double (&g1u)[P + 1], double (&g0v)[P + 1], double (&g1v)[P + 1]) {
-    constexpr double third = 1.0 / 3.0, sixth = 1.0 / 6.0;
-    double C[P + 1];
+                                                double coef, const double (&dc)[P + 1], const double (&s_u)[P + 1],
+                                                const double (&d_u)[P + 1], const double (&s_v)[P + 1],
+                                                const double (&d_v)[P + 1], double (&gdc)[P + 1],
+                                                double (&gsu)[P + 1], double (&gdu)[P + 1], double (&gsv)[P + 1],
+                                                double (&gdv)[P + 1]) {
+    constexpr double kSqrt12 = 3.4641016151377546;
+    double C[P], M[P];
     double acc = 0.0;
 #pragma unroll
-    for (int a = 0; a <= P; ++a) {
-        acc += s1c[a] - s0c[a];
-        C[a] = (a < lc - 1) ? acc : 0.0;   // the last running-sum point is not deposited
+    for (int a = 0; a < P; ++a) {
+        acc += dc[a];
+        C[a] = (a < lc - 1) ? coef * kSqrt12 * acc : 0.0;   // the last running-sum point is not deposited
+        M[a] = 0.0;
     }
-    double M[P + 1];
-#pragma unroll
-    for (int a = 0; a <= P; ++a) M[a] = 0.0;
-    double G = 0.0;
+#pragma unroll 1
     for (int b = 0; b < lv; ++b) {
-        const double s0b = pick(s0v, b), s1b = pick(s1v, b);
-        double dv0 = 0.0, dv1 = 0.0;
+        const double sb = pick(s_v, b), db = pick(d_v, b);
+        double ts = 0.0, td = 0.0;
 #pragma unroll
         for (int a = 0; a <= P; ++a) {
             if (a >= lu) break;
-            const double W = third * s0u[a] * s0b + sixth * s1u[a] * s0b + sixth * s0u[a] * s1b + third * s1u[a] * s1b;
+            const double W = s_u[a] * sb + d_u[a] * db;
             double T = 0.0;
             const LT *row = lam + b * sv + a * su;
 #pragma unroll
@@ -256,29 +241,28 @@ __device__ __forceinline__ double esirkepov_adj(const LT *lam, int sc, int su, i
                 T += C[q] * l;
                 M[q] += l * W;
             }
-            G += T * W;
-            g0u[a] += coef * T * (third * s0b + sixth * s1b);
-            g1u[a] += coef * T * (sixth * s0b + third * s1b);
-            dv0 += T * (third * s0u[a] + sixth * s1u[a]);
-            dv1 += T * (sixth * s0u[a] + third * s1u[a]);
+            gsu[a] += T * sb;
+            gdu[a] += T * db;
+            ts += T * s_u[a];
+            td += T * d_u[a];
         }
-        // add into g0v[b], g1v[b] for a run-time b
+        // add into gsv[b], gdv[b] for a run-time b
 #pragma unroll
         for (int q = 0; q <= P; ++q)
             if (q == b) {
-                g0v[q] += coef * dv0;
-                g1v[q] += coef * dv1;
+                gsv[q] += ts;
+                gdv[q] += td;
             }
     }
-    // dG/dds(q') = coef * sum_{q >= q'} M(q); ds = s1 - s0
-    double suf = 0.0;
+    // dG/dds(q') = coef * sum_{q >= q'} M(q)
+    double suf = 0.0, G = 0.0;
 #pragma unroll
-    for (int q = P; q >= 0; --q) {
+    for (int q = P - 1; q >= 0; --q) {
+        G += C[q] * M[q];
         suf += M[q];
-        g1c[q] += coef * suf;
-        g0c[q] -= coef * suf;
+        gdc[q] += coef * kSqrt12 * suf;
     }
-    return coef * G;
+    return G;
 }
 
 template <typename real>
@@ -379,22 +363,16 @@ __device__ __forceinline__ bool adj_particle(const AdjPushArgs<real> &a, long lo
         gather_grad<real, P, LDG>(fv[4], id[0] - H, ip[1] - H, id[2] - H, wd[0], wp[1], wd[2], gd[0], gp[1], gd[2], ev[4], eg[4]);
         gather_grad<real, P, LDG>(fv[5], id[0] - H, id[1] - H, ip[2] - H, wd[0], wd[1], wp[2], gd[0], gd[1], gp[2], ev[5], eg[5]);
         }
-        // ---- Boris Jacobian: three passes of three tangents (p, e, b) -----
+        // ---- Boris: values only here (the displacement fixes the new
+        // position); they are formed again for the transpose, after the deposit
+        // adjoint ------------------------------------------------------------
         const real pin[3] = {a.px[p], a.py[p], a.pz[p]};
-        // values only here (the displacement fixes the new position); the
-        // tangents are formed after the deposit adjoint, contracted at once
         real disp_v[3];
         {
-            Dual<real, 1> P_[3], E_[3], B_[3], pn[3], ds[3];
+            Boris<real> v;
+            boris_values<real>(pin, ev, ev + 3, a.qm, v);
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                P_[d] = dconst<real, 1>(pin[d]);
-                E_[d] = dconst<real, 1>(ev[d]);
-                B_[d] = dconst<real, 1>(ev[3 + d]);
-            }
-            boris_dual<real, 1>(P_, E_, B_, a.qm, a.dt_d, pn, ds);
-#pragma unroll
-            for (int o = 0; o < 3; ++o) disp_v[o] = ds[o].v;
+            for (int o = 0; o < 3; ++o) disp_v[o] = v.pn[o] * v.ig * a.dt_d[o];
         }
         // ---- new position, as the forward deposit forms it ----------------
         int i2[3];
@@ -423,19 +401,24 @@ __device__ __forceinline__ bool adj_particle(const AdjPushArgs<real> &a, long lo
             return false;
         }
         // ---- deposit adjoint ----------------------------------------------
-        double s0[3][P + 1], s1[3][P + 1];   // weights on the common span
-        double g0[3][P + 1], g1[3][P + 1];   // dG1 / d(weights)
+        constexpr double kInvSqrt12 = 0.28867513459481287;
+        double ss[3][P + 1], sd[3][P + 1];   // s and d of each axis on the common span
+        double gs[3][P + 1], gd[3][P + 1];   // dG1 / d(s, d)
         int base[3], len[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            double w0[P], w1[P];
+            double w0[P], w1[P], u0[P + 1], u1[P + 1];
             shape_weights(d0[d], w0);
             shape_weights(d2[d], w1);
-            span_pair<double, P>(ip[d], w0, i2[d], w1, s0[d], s1[d]);
+            span_pair<double, P>(ip[d], w0, i2[d], w1, u0, u1);
             base[d] = min(ip[d], i2[d]) - H;
             len[d] = P + abs(i2[d] - ip[d]);
 #pragma unroll
-            for (int q = 0; q <= P; ++q) g0[d][q] = g1[d][q] = 0.0;
+            for (int q = 0; q <= P; ++q) {
+                ss[d][q] = 0.5 * (u0[q] + u1[q]);
+                sd[d][q] = kInvSqrt12 * (u1[q] - u0[q]);
+                gs[d][q] = gd[d][q] = 0.0;
+            }
         }
         const double qd = (double)a.charge;
         double G1 = 0.0;
@@ -446,14 +429,14 @@ __device__ __forceinline__ bool adj_particle(const AdjPushArgs<real> &a, long lo
             const real *lbuf = lj[comp].at(base[2], base[1], base[0]);
             const int sX = 1, sY = lj[comp].sy, sZ = lj[comp].sz;
             if (comp == 0)
-                G1 += esirkepov_adj<P, LDG>(lbuf, sX, sY, sZ, len[0], len[1], len[2], -qd * a.d_dt[0], s0[0], s1[0],
-                                       s0[1], s1[1], s0[2], s1[2], g0[0], g1[0], g0[1], g1[1], g0[2], g1[2]);
+                G1 += esirkepov_adj<P, LDG>(lbuf, sX, sY, sZ, len[0], len[1], len[2], -qd * a.d_dt[0], sd[0], ss[1], sd[1],
+                                            ss[2], sd[2], gd[0], gs[1], gd[1], gs[2], gd[2]);
             else if (comp == 1)
-                G1 += esirkepov_adj<P, LDG>(lbuf, sY, sX, sZ, len[1], len[0], len[2], -qd * a.d_dt[1], s0[1], s1[1],
-                                       s0[0], s1[0], s0[2], s1[2], g0[1], g1[1], g0[0], g1[0], g0[2], g1[2]);
+                G1 += esirkepov_adj<P, LDG>(lbuf, sY, sX, sZ, len[1], len[0], len[2], -qd * a.d_dt[1], sd[1], ss[0], sd[0],
+                                            ss[2], sd[2], gd[1], gs[0], gd[0], gs[2], gd[2]);
             else
-                G1 += esirkepov_adj<P, LDG>(lbuf, sZ, sX, sY, len[2], len[0], len[1], -qd * a.d_dt[2], s0[2], s1[2],
-                                       s0[0], s1[0], s0[1], s1[1], g0[2], g1[2], g0[0], g1[0], g0[1], g1[1]);
+                G1 += esirkepov_adj<P, LDG>(lbuf, sZ, sX, sY, len[2], len[0], len[1], -qd * a.d_dt[2], sd[2], ss[0], sd[0],
+                                            ss[1], sd[1], gd[2], gs[0], gd[0], gs[1], gd[1]);
         }
         const double wgt = (double)a.w[p];
         a.lw[p] += G1;
@@ -467,39 +450,20 @@ __device__ __forceinline__ bool adj_particle(const AdjPushArgs<real> &a, long lo
             double s_0 = 0.0, s_1 = 0.0;
 #pragma unroll
             for (int q = 0; q <= P; ++q) {
-                s_0 += g0[d][q] * t0[q];
-                s_1 += g1[d][q] * t1[q];
+                const double hs = 0.5 * gs[d][q], hd = kInvSqrt12 * gd[d][q];
+                s_0 += (hs - hd) * t0[q];
+                s_1 += (hs + hd) * t1[q];
             }
             dGx0[d] = wgt * s_0;
             dGx1[d] = wgt * s_1;
         }
-        // ---- chain rule: lin = J^T (lp', lx') with J = d(p', disp) / d(p, e,
-        // b), one forward-mode pass of three tangents per input group ------
+        // ---- chain rule: lin = J^T (lp', lx') ----------------------------
         const real lxn[3] = {a.lx[p] + (real)dGx1[0], a.ly[p] + (real)dGx1[1], a.lz[p] + (real)dGx1[2]};
         const real lpn[3] = {a.lpx[p], a.lpy[p], a.lpz[p]};
-#pragma unroll
-        for (int pass = 0; pass < 3; ++pass) {
-            Dual<real, 3> P_[3], E_[3], B_[3], pn[3], ds[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                P_[d] = dconst<real, 3>(pin[d]);
-                E_[d] = dconst<real, 3>(ev[d]);
-                B_[d] = dconst<real, 3>(ev[3 + d]);
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                if (pass == 0) P_[d].d[d] = real(1);
-                if (pass == 1) E_[d].d[d] = real(1);
-                if (pass == 2) B_[d].d[d] = real(1);
-            }
-            boris_dual<real, 3>(P_, E_, B_, a.qm, a.dt_d, pn, ds);
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                real s = 0;
-#pragma unroll
-                for (int o = 0; o < 3; ++o) s += lpn[o] * pn[o].d[t] + lxn[o] * ds[o].d[t];
-                lin[3 * pass + t] = s;
-            }
+        {
+            Boris<real> v;
+            boris_values<real>(pin, ev, ev + 3, a.qm, v);
+            boris_transpose<real>(v, a.qm, a.dt_d, lpn, lxn, lin);
         }
         real lxo[3];
 #pragma unroll
@@ -586,7 +550,8 @@ __global__ void __launch_bounds__(128) adj_push_kernel(AdjPushArgs<real> a) {
 // forward push, i.e. sorted by tile at the last sort; with each sort the tape
 // also keeps the tile boundaries of that order.  One CTA per tile:
 //   1. stages the tape's six field components over the tile's gather box
-//      and the three J adjoints over its deposit box in shared memory;
+//      and the three J adjoints over its deposit box in shared memory; then,
+//      for as many particles at a time as the scratch holds,
 //   2. runs each particle's push adjoint from shared memory, keeping the
 //      adjoints of its gathered E and B (six values) and their largest
 //      magnitude per component;
@@ -594,14 +559,22 @@ __global__ void __launch_bounds__(128) adj_push_kernel(AdjPushArgs<real> a) {
 //      fixed-point shared accumulators (20-bit limbs as the forward deposit,
 //      scaled so that the largest value fits), then flushes them with one
 //      pass of global atomics.
-// Particles that left their tile since the sort, and tiles with more
-// particles than the scratch holds, go to the global kernel afterwards.
+// Particles that left their tile since the sort go to the global kernel
+// afterwards.
+//
+// What bounds it: latency.  About 15 k instructions per 32 particles (scatter
+// 30 %, Esirkepov transpose in FP64 27 %, gather with gradients 20 %) issue at
+// 0.34 of the rate, two warps per scheduler at 255 registers.  384 or 512
+// threads spill and are no faster (FP32 592 and 618 against 593 us, FP64 352
+// and 423 against 339 us, 48 x 32 x 32 and 32 x 24 x 24 cells with 8 per cell),
+// nor are two FP32 CTAs of 128 threads (565 against 559 us).
 
 struct AdjTileGeom {
     int T, nt[3];
+    int nodes;               // 1: tiles of nodes, 0: tiles of cells
     int GE, DE;
     int gsy, gsz, gsize, dsy, dsz, dsize;
-    int cap;                 // particles per tile the shared scratch holds
+    int cap;                 // particles the shared scratch holds
 };
 
 template <typename real>
@@ -625,9 +598,10 @@ __device__ __forceinline__ void fixed_add(unsigned *a, int lstride, real q) {
 
 // TT: the tile edge as a compile-time constant (0: from tg), which makes
 // every shared-box stride a constant.
+constexpr int kAdjThreads = 256;
 template <typename real, int P, int TT>
-__global__ void __launch_bounds__(256, 1) adj_tile_kernel(AdjPushArgs<real> a, AdjTileGeom tg, const unsigned *toffs,
-                                                          int *strag, unsigned long long *nstrag) {
+__global__ void __launch_bounds__(kAdjThreads, 1) adj_tile_kernel(const __grid_constant__ AdjPushArgs<real> a, AdjTileGeom tg,
+                                                          const unsigned *toffs, int *strag, unsigned long long *nstrag) {
     AdjTileGeom t = tg;
     if constexpr (TT > 0) {
         constexpr int ge = TT + 2 * (P / 2) + 1, de = TT + 2 * (P / 2) + 3;
@@ -637,7 +611,7 @@ __global__ void __launch_bounds__(256, 1) adj_tile_kernel(AdjPushArgs<real> a, A
         t.gsy = gy; t.gsz = gz; t.gsize = ge * gz;
         t.dsy = dy; t.dsz = dz; t.dsize = de * dz;
     }
-    constexpr int H = P / 2, NL = adj_limbs<real>();
+    constexpr int H = P / 2, NL = adj_limbs<real>(), NT = kAdjThreads;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geom &g = a.g;
     const int T = t.T, GE = t.GE, DE = t.DE, GS = t.gsize, DS = t.dsize;
@@ -653,144 +627,166 @@ __global__ void __launch_bounds__(256, 1) adj_tile_kernel(AdjPushArgs<real> a, A
     int gO[3], dO[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        gO[d] = t0[d] + g.mem - 1 - H;
+        // the lowest dual stencil starts a point lower where tiles hold nodes
+        gO[d] = t0[d] + g.mem - 1 - H - t.nodes;
         dO[d] = t0[d] + g.mem - 2 - H;
     }
     long long pa = toffs[tile], pb = toffs[tile + 1];
     pb = pb < a.n ? pb : a.n;
-    if (pa > pb) pa = pb;
-    const long long m = pb - pa;
-    if (m == 0) return;
-    const bool use_smem = m <= t.cap;
-    if (!use_smem) {
-        for (long long i = threadIdx.x; i < m; i += blockDim.x) {
-            const long long p = pa + i;
-            if (!(a.dead && a.dead[p])) strag[atomicAdd(nstrag, 1ull)] = (int)p;
-        }
-        return;
-    }
+    if (pa >= pb) return;
+    const int m_all = (int)(pb - pa);
     const int G2 = GE * GE, G3 = G2 * GE, D2 = DE * DE, D3 = D2 * DE;
-    for (int e = threadIdx.x; e < 6 * G3; e += blockDim.x) {
-        int c = e / G3, l = e - c * G3;
-        int lz = l / G2, r = l - lz * G2, ly = r / GE, lx = r - ly * GE;
-        int x = gO[0] + lx, y = gO[1] + ly, z = gO[2] + lz;
-        real v = 0;
-        if (x >= 0 && x < g.f[0] && y >= 0 && y < g.f[1] && z >= 0 && z < g.f[2]) v = __ldg(a.f[c] + g.fi(z, y, x));
-        sf[c * GS + lz * t.gsz + ly * t.gsy + lx] = v;
+    for (int l = threadIdx.x; l < G3; l += NT) {
+        const int lz = l / G2, r = l - lz * G2, ly = r / GE, lx = r - ly * GE;
+        const int x = gO[0] + lx, y = gO[1] + ly, z = gO[2] + lz;
+        const bool in = x >= 0 && x < g.f[0] && y >= 0 && y < g.f[1] && z >= 0 && z < g.f[2];
+        const int src = in ? g.fi(z, y, x) : 0;
+        real *dst = sf + lz * t.gsz + ly * t.gsy + lx;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) cp_async<sizeof(real)>(dst + c * GS, a.f[c] + src, in ? (int)sizeof(real) : 0);
     }
-    for (int e = threadIdx.x; e < 3 * D3; e += blockDim.x) {
-        int c = e / D3, l = e - c * D3;
-        int lz = l / D2, r = l - lz * D2, ly = r / DE, lx = r - ly * DE;
-        int x = dO[0] + lx, y = dO[1] + ly, z = dO[2] + lz;
-        real v = 0;
-        if (x >= -1 && x <= g.f[0] && y >= -1 && y <= g.f[1] && z >= -1 && z <= g.f[2]) v = __ldg(a.lj[c] + g.ri(z, y, x));
-        sl[c * DS + lz * t.dsz + ly * t.dsy + lx] = v;
+    for (int l = threadIdx.x; l < D3; l += NT) {
+        const int lz = l / D2, r = l - lz * D2, ly = r / DE, lx = r - ly * DE;
+        const int x = dO[0] + lx, y = dO[1] + ly, z = dO[2] + lz;
+        const bool in = x >= -1 && x <= g.f[0] && y >= -1 && y <= g.f[1] && z >= -1 && z <= g.f[2];
+        const int src = in ? g.ri(z, y, x) : 0;
+        real *dst = sl + lz * t.dsz + ly * t.dsy + lx;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cp_async<sizeof(real)>(dst + c * DS, a.lj[c] + src, in ? (int)sizeof(real) : 0);
     }
-    for (int e = threadIdx.x; e < 6 * NL * GS; e += blockDim.x) acc[e] = 0u;
+    cp_async_commit();
+    for (int e = threadIdx.x; e < 6 * NL * GS; e += NT) acc[e] = 0u;
     if (threadIdx.x < 6) smax[threadIdx.x] = 0u;
+    cp_async_wait_all();
     __syncthreads();
     View<const real> fv[6], lj[3];
 #pragma unroll
     for (int c = 0; c < 6; ++c) fv[c] = View<const real>{sf + c * GS, t.gsy, t.gsz, -(gO[2] * t.gsz + gO[1] * t.gsy + gO[0])};
 #pragma unroll
     for (int c = 0; c < 3; ++c) lj[c] = View<const real>{sl + c * DS, t.dsy, t.dsz, -(dO[2] * t.dsz + dO[1] * t.dsy + dO[0])};
-    // 2. the particles' push adjoints
-    for (long long i = threadIdx.x; i < m; i += blockDim.x) {
-        const long long p = pa + i;
-        flag[i] = 0;
-        if (a.dead && a.dead[p]) continue;
-        int idl[3];   // dual index per axis (the cell's lower primal point)
-        if constexpr (sizeof(real) == 8) {
-            idl[0] = (int)(a.x[p] - (double)(1 - g.mem));
-            idl[1] = (int)(a.y[p] - (double)(1 - g.mem));
-            idl[2] = (int)(a.z[p] - (double)(1 - g.mem));
-        } else {
-            int cc[3];
-            a.cp.unpack(a.cell[p], cc[0], cc[1], cc[2]);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) idl[d] = cc[d] + g.mem - 1;
-        }
-        bool inside = true;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) inside = inside && idl[d] >= t0[d] + g.mem - 1 && idl[d] < t0[d] + g.mem - 1 + T;
-        if (!inside) {
-            strag[atomicAdd(nstrag, 1ull)] = (int)p;
-            continue;
-        }
-        real lin[9];
-        if (!adj_particle<real, P, false>(a, p, fv, lj, lin)) continue;
-        if (!a.scatter_fields) continue;
-        flag[i] = 1;
-        // per component the largest magnitude of the tile: reduced over the
-        // warp's active lanes first, one shared atomic per warp
-        const unsigned am = __activemask();
-        const bool leader = (threadIdx.x & 31) == __ffs(am) - 1;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            slin[c * t.cap + i] = lin[3 + c];
-            const unsigned mag = __reduce_max_sync(am, __float_as_uint((float)fabs(lin[3 + c])));
-            if (leader) atomicMax(smax + c, mag);
-        }
-    }
-    if (!a.scatter_fields) return;
-    __syncthreads();
-    // 3. field adjoints into fixed point, then one flush
-    const double lim = sizeof(real) == 8 ? 2251799813685248.0 /* 2^51 */ : 2147483648.0 /* 2^31 */;
-    real scale[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        const double mx = (double)__uint_as_float(smax[c]);
-        scale[c] = mx > 0.0 ? (real)(lim / (1.01 * mx)) : real(0);
-    }
-    for (long long i = threadIdx.x; i < m; i += blockDim.x) {
-        if (!flag[i]) continue;
-        int ip[3], id[3];
-        real wp[3][P], wd[3][P];
-        gather_stencils<real, P>(a, pa + i, ip, id, wp, wd);
-        // stencil origin per component (Yee staggering as in the gather)
-        const int o[6][3] = {{id[0], ip[1], ip[2]}, {ip[0], id[1], ip[2]}, {ip[0], ip[1], id[2]},
-                             {ip[0], id[1], id[2]}, {id[0], ip[1], id[2]}, {id[0], id[1], ip[2]}};
 #pragma unroll 1
-        for (int c = 0; c < 6; ++c) {
-            const real q = slin[c * t.cap + i] * scale[c];
-            if (q == real(0)) continue;
-            // dual axes: Ex x; Ey y; Ez z; Bx y, z; By x, z; Bz x, y
-            const bool dx_ = c == 0 || c == 4 || c == 5, dy_ = c == 1 || c == 3 || c == 5,
-                       dz_ = c == 2 || c == 3 || c == 4;
-            real wx[P], wy[P], wz[P];
+    for (int first = 0; first < m_all; first += t.cap, pa += t.cap) {
+        const int m = min(t.cap, m_all - first);
+        // 2. the particles' push adjoints
+#pragma unroll 1
+        for (int i = threadIdx.x; i < m; i += NT) {
+            const long long p = pa + i;
+            flag[i] = 0;
+            if (a.dead && a.dead[p]) continue;
+            // dual index (the cell's lower primal point), or the node, per axis
+            int at[3];
+            if constexpr (sizeof(real) == 8) {
+                const double half = t.nodes ? 0.5 : 0.0;
+                at[0] = (int)(a.x[p] - (double)(1 - g.mem) + half);
+                at[1] = (int)(a.y[p] - (double)(1 - g.mem) + half);
+                at[2] = (int)(a.z[p] - (double)(1 - g.mem) + half);
+            } else {
+                int cc[3];
+                a.cp.unpack(a.cell[p], cc[0], cc[1], cc[2]);
+                const float o[3] = {a.ox[p], a.oy[p], a.oz[p]};
 #pragma unroll
-            for (int q2 = 0; q2 < P; ++q2) {
-                wx[q2] = dx_ ? wd[0][q2] : wp[0][q2];
-                wy[q2] = dy_ ? wd[1][q2] : wp[1][q2];
-                wz[q2] = dz_ ? wd[2][q2] : wp[2][q2];
+                for (int d = 0; d < 3; ++d) at[d] = cc[d] + g.mem - 1 + (t.nodes && o[d] >= 0.5f ? 1 : 0);
             }
-            unsigned *ac = acc + c * NL * GS;
-            const int b0 = (o[c][2] - H - gO[2]) * t.gsz + (o[c][1] - H - gO[1]) * t.gsy + (o[c][0] - H - gO[0]);
+            bool inside = true;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) inside = inside && at[d] >= t0[d] + g.mem - 1 && at[d] < t0[d] + g.mem - 1 + T;
+            if (!inside) {
+                strag[atomicAdd(nstrag, 1ull)] = (int)p;
+                continue;
+            }
+            real lin[9];
+            if (!adj_particle<real, P, false>(a, p, fv, lj, lin)) continue;
+            if (!a.scatter_fields) continue;
+            flag[i] = 1;
+            // per component the largest magnitude of the tile: reduced over the
+            // warp's active lanes first, one shared atomic per warp
+            const unsigned am = __activemask();
+            const bool leader = (threadIdx.x & 31) == __ffs(am) - 1;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                slin[c * t.cap + i] = lin[3 + c];
+                const unsigned mag = __reduce_max_sync(am, __float_as_uint((float)fabs(lin[3 + c])));
+                if (leader) atomicMax(smax + c, mag);
+            }
+        }
+        if (!a.scatter_fields) continue;
+        __syncthreads();
+        // 3. field adjoints into fixed point, then one flush
+        const double lim = sizeof(real) == 8 ? 2251799813685248.0 /* 2^51 */ : 2147483648.0 /* 2^31 */;
+        real scale[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            const double mx = (double)__uint_as_float(smax[c]);
+            scale[c] = mx > 0.0 ? (real)(lim / (1.01 * mx)) : real(0);
+        }
+        // Sorted by node, neighbouring particles add to the same points: the
+        // lanes of a warp take particles m / 32 apart.
+        const int step = t.nodes ? (m + 31) >> 5 : 1;
+        const int lane = threadIdx.x & 31, nb = (m + 31) >> 5;
 #pragma unroll 1
-            for (int k = 0; k < P; ++k) {
-                const real qk = q * pick(wz, k);
+        for (int b = threadIdx.x >> 5; b < nb; b += NT / 32) {
+            const int i = t.nodes ? lane * step + b : b * 32 + lane;
+            if (i >= m || !flag[i]) continue;
+            int ip[3], id[3];
+            real wp[3][P], wd[3][P];
+            gather_stencils<real, P>(a, pa + i, ip, id, wp, wd);
+#pragma unroll 1
+            for (int c = 0; c < 6; ++c) {
+                const real q = slin[c * t.cap + i] * (c == 0 ? scale[0] : c == 1 ? scale[1] : c == 2 ? scale[2] : c == 3 ? scale[3]
+                                                      : c == 4 ? scale[4] : scale[5]);
+                if (q == real(0)) continue;
+                // dual axes (Yee staggering as in the gather): Ex x; Ey y; Ez z; Bx y, z; By x, z; Bz x, y
+                const bool dx_ = c == 0 || c == 4 || c == 5, dy_ = c == 1 || c == 3 || c == 5,
+                           dz_ = c == 2 || c == 3 || c == 4;
+                real wx[P], wy[P], wz[P];
 #pragma unroll
-                for (int j = 0; j < P; ++j) {
-                    const real qj = qk * wy[j];
+                for (int q2 = 0; q2 < P; ++q2) {
+                    wx[q2] = dx_ ? wd[0][q2] : wp[0][q2];
+                    wy[q2] = dy_ ? wd[1][q2] : wp[1][q2];
+                    wz[q2] = dz_ ? wd[2][q2] : wp[2][q2];
+                }
+                unsigned *ac = acc + c * NL * GS;
+                const int b0 = ((dz_ ? id[2] : ip[2]) - H - gO[2]) * t.gsz + ((dy_ ? id[1] : ip[1]) - H - gO[1]) * t.gsy +
+                               ((dx_ ? id[0] : ip[0]) - H - gO[0]);
+#pragma unroll 1
+                for (int k = 0; k < P; ++k) {
+                    const real qk = q * pick(wz, k);
 #pragma unroll
-                    for (int ii = 0; ii < P; ++ii) fixed_add<real, NL>(ac + b0 + k * t.gsz + j * t.gsy + ii, GS, qj * wx[ii]);
+                    for (int j = 0; j < P; ++j) {
+                        const real qj = qk * wy[j];
+#pragma unroll
+                        for (int ii = 0; ii < P; ++ii)
+                            fixed_add<real, NL>(ac + b0 + k * t.gsz + j * t.gsy + ii, GS, qj * wx[ii]);
+                    }
                 }
             }
         }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 6 * G3; e += blockDim.x) {
-        int c = e / G3, l = e - c * G3;
-        if (scale[c] == real(0)) continue;
-        int lz = l / G2, r = l - lz * G2, ly = r / GE, lx = r - ly * GE;
-        const unsigned *q = acc + c * NL * GS + lz * t.gsz + ly * t.gsy + lx;
-        long long tot;
-        if constexpr (NL == 2) tot = ((long long)(int)q[GS] << 20) + (long long)q[0];
-        else tot = ((long long)(int)q[2 * GS] << 40) + ((long long)q[GS] << 20) + (long long)q[0];
-        if (tot == 0) continue;
-        int x = gO[0] + lx, y = gO[1] + ly, z = gO[2] + lz;
-        if (x >= 0 && x < g.f[0] && y >= 0 && y < g.f[1] && z >= 0 && z < g.f[2])
-            atomic_add(a.lf[c] + g.fi(z, y, x), (real)((double)tot / (double)scale[c]));
+        __syncthreads();
+        const bool more = first + t.cap < m_all;
+        double inv[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) inv[c] = scale[c] > real(0) ? 1.0 / (double)scale[c] : 0.0;
+        if (threadIdx.x < 6) smax[threadIdx.x] = 0u;
+        for (int l = threadIdx.x; l < G3; l += NT) {
+            const int lz = l / G2, r = l - lz * G2, ly = r / GE, lx = r - ly * GE;
+            const int x = gO[0] + lx, y = gO[1] + ly, z = gO[2] + lz;
+            const bool in = x >= 0 && x < g.f[0] && y >= 0 && y < g.f[1] && z >= 0 && z < g.f[2];
+            const int dst = in ? g.fi(z, y, x) : 0;
+            unsigned *q = acc + lz * t.gsz + ly * t.gsy + lx;
+#pragma unroll
+            for (int c = 0; c < 6; ++c, q += NL * GS) {
+                long long tot;
+                if constexpr (NL == 2) tot = ((long long)(int)q[GS] << 20) + (long long)q[0];
+                else tot = ((long long)(int)q[2 * GS] << 40) + ((long long)q[GS] << 20) + (long long)q[0];
+                if (tot == 0) continue;
+                if (more) {
+#pragma unroll
+                    for (int n = 0; n < NL; ++n) q[n * GS] = 0u;
+                }
+                if (in) atomic_add(a.lf[c] + dst, (real)((double)tot * inv[c]));
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1374,13 +1370,16 @@ static void adj_push_launch(pic_ctx *c, AdjState *A, const Blob &b, int kind, in
         AdjTileGeom tg{};
         tg.T = c->tile;
         for (int d = 0; d < 3; ++d) tg.nt[d] = c->ntile[d];
+        tg.nodes = c->node_tiles ? 1 : 0;
         tg.GE = bx.GE; tg.DE = bx.DE;
         tg.gsy = bx.gsy; tg.gsz = bx.gsz; tg.gsize = bx.gsize;
         tg.dsy = bx.dsy; tg.dsz = bx.dsz; tg.dsize = bx.dsize;
+        // scratch for 10 (FP64) or 18 (FP32) particles per cell of the default
+        // tile, at most 4095 (the limbs): beyond, the tile takes several rounds
         const size_t rs = sizeof(real), nl = adj_limbs<real>();
         const size_t fixed = (6 * (size_t)bx.gsize + 3 * (size_t)bx.dsize) * rs + (6 * nl * bx.gsize + 8) * 4;
         const size_t budget = 227 * 1024;
-        tg.cap = fixed + 64 < budget ? (int)std::min<size_t>(4095, (budget - fixed - 64) / (6 * rs + 1)) : 0;
+        tg.cap = fixed + 64 < budget ? (int)std::min<size_t>(rs == 8 ? 640 : 1152, (budget - fixed - 64) / (6 * rs + 1)) : 0;
         const size_t smem = fixed + (size_t)tg.cap * (6 * rs + 1);
         const int ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
         cudaMemsetAsync(c->d_nstrag + kind, 0, sizeof(unsigned long long), c->stream);
@@ -1389,10 +1388,10 @@ static void adj_push_launch(pic_ctx *c, AdjState *A, const Blob &b, int kind, in
             const unsigned *toffs = (const unsigned *)blob_part(b, b.toff_part[kind]);
             if (c->tile == 4) {   // the default edge: strides as constants
                 cudaFuncSetAttribute(adj_tile_kernel<real, P, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                adj_tile_kernel<real, P, 4><<<ntiles, 256, smem, c->stream>>>(a, tg, toffs, s.strag, c->d_nstrag + kind);
+                adj_tile_kernel<real, P, 4><<<ntiles, kAdjThreads, smem, c->stream>>>(a, tg, toffs, s.strag, c->d_nstrag + kind);
             } else {
                 cudaFuncSetAttribute(adj_tile_kernel<real, P, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                adj_tile_kernel<real, P, 0><<<ntiles, 256, smem, c->stream>>>(a, tg, toffs, s.strag, c->d_nstrag + kind);
+                adj_tile_kernel<real, P, 0><<<ntiles, kAdjThreads, smem, c->stream>>>(a, tg, toffs, s.strag, c->d_nstrag + kind);
             }
             a.idx = s.strag;
             a.nidx = c->d_nstrag + kind;

@@ -523,7 +523,7 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     // of the reverse sweep (each sort's permutation goes on the tape).
     c->sort_interval = p.sort_interval > 0 ? p.sort_interval : (p.adjoint ? 1 : 4);
     if (c->tile > 0) {
-        c->node_tiles = node_tiles_for(c->tile, p.adjoint != 0, c->order);
+        c->node_tiles = node_tiles_for(c->tile, c->order);
         // cells 0 .. n-1, or nodes 0 .. n
         for (int d = 0; d < 3; ++d) c->ntile[d] = (n[d] + (c->node_tiles ? 1 : 0) + c->tile - 1) / c->tile;
         c->keys_per_tile = (long long)c->tile * c->tile * c->tile * (c->node_tiles ? 1 : kOctants);
@@ -1047,7 +1047,7 @@ int pic_initial_push(pic_ctx *c) {
 // between them writes a field): both are then done here in one pass.
 static int run_one_step(pic_ctx *c, bool rho_observed, bool e_first, bool e_next) {
     c->step += 1;
-    c->rho_skip = !rho_observed && !c->p.adjoint;
+    c->rho_skip = !rho_observed;
     const unsigned rings = c->rho_skip ? 7u : 31u;
     int r;
     if ((r = pic_radiating_boundary(c, 1, 0, c->step))) return r;

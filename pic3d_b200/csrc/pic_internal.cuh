@@ -244,7 +244,7 @@ struct pic_ctx {
     int sort_interval = 4;
     // rho is observable only between ABI calls: the intermediate steps of
     // one pic_run_steps call neither clear, deposit nor fold it (set while
-    // such a step runs; never in adjoint mode, whose checkpoints copy rho)
+    // such a step runs; checkpoints, which copy rho, are saved between calls)
     bool rho_skip = false;
     int steps_since_sort = 0;
     int step = 0;

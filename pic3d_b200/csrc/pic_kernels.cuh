@@ -84,7 +84,7 @@ TileBoxes tile_boxes(const pic_ctx *c);
 size_t tile_smem_bytes(const pic_ctx *c);
 
 // tile_mma_kernels.cu
-bool node_tiles_for(int tile, bool adjoint, int order);   // whether a context uses tiles of nodes
+bool node_tiles_for(int tile, int order);   // whether a context uses tiles of nodes
 size_t node_tile_smem_bytes(const pic_ctx *c);
 void launch_node_tile_kernel(pic_ctx *c, int mask, bool spin);
 

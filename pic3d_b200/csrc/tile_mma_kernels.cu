@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(NodeTile<real, P>::kThreads, NodeTile<real, P>
         int row = -1;          // its row (y + 4 z of the node) if it takes part in the matrix products
         int geo = 0;           // lower node + 1 per axis (3 bits each), move in nodes + 1 per axis (2 bits each)
         Moved<real> mv;
-        if (i < m[k]) {
+        // (adjoint contexts: removed particles stay, dead)
+        if (i < m[k] && !(a.dead && a.dead[loc.x])) {
             const long long p = loc.x;
             const int home = loc.y;
             PartIn<real> in;
@@ -540,9 +541,8 @@ void node_tile_push(pic_ctx *c, int mask) {
 // 7.08 -> 4.07 ms, FP32 3.72 -> 2.42 ms.  At 2nd order the factors of its
 // products cost more to make (FP32 1.23 ms) than a particle's 54 points to
 // scatter (1.01 ms): tile_node_kernels.cu sums them per node instead.  Other
-// edges and adjoint contexts (whose reverse sweep shares the tiles) keep the
-// tiles of cells of tile_kernels.cu.
-bool node_tiles_for(int tile, bool adjoint, int order) { return tile == 4 && !adjoint && (order == 2 || order == 4); }
+// edges keep the tiles of cells of tile_kernels.cu.
+bool node_tiles_for(int tile, int order) { return tile == 4 && (order == 2 || order == 4); }
 
 size_t node_tile_smem_bytes(const pic_ctx *c) {
     if (c->order == 2) return node_sum_smem_bytes(c);
