@@ -68,7 +68,6 @@ void free_arrays(PartArrays &a) {
 void free_species(Species &s) {
     free_arrays(s.a);
     free_arrays(s.b);
-    if (s.d_count) cudaFree(s.d_count);
     if (s.keys) cudaFree(s.keys);
     if (s.strag) cudaFree(s.strag);
     if (s.dead) cudaFree(s.dead);
@@ -130,7 +129,7 @@ int alloc_species(pic_ctx *c, int kind, int64_t cap, bool spin) {
         }
     }
     if (cap > 0) r = r ? r : dalloc(c, &s.strag, 2 * n * sizeof(int));
-    r = r ? r : dalloc(c, &s.d_count, sizeof(long long));
+    s.d_count = c->d_state + 1 + kind;
     if (c->p.adjoint && cap > 0) r = r ? r : dalloc(c, &s.dead, n);
     if (c->p.adjoint && c->tile > 0 && cap > 0) {
         r = r ? r : dalloc(c, &s.orig, n * sizeof(int));
@@ -290,9 +289,10 @@ static int staged_h2d(pic_ctx *c, void *dev, const void *host, size_t bytes) {
     int r = ensure_pinned(c, kPinRecords);
     if (r) return r;
     const size_t chunk = (size_t)kPinRecords * 144;
-    for (size_t off = 0, i = 0; off < bytes; off += chunk, ++i) {
+    for (size_t off = 0; off < bytes; off += chunk) {
         const size_t m = std::min(chunk, bytes - off);
-        const int b = (int)(i & 1);
+        const int b = c->pin_next;
+        c->pin_next ^= 1;
         CK(cudaEventSynchronize(c->pin_ev[b]));
         par_memcpy(c->h_pin[b], (const char *)host + off, m);
         CK(cudaMemcpyAsync((char *)dev + off, c->h_pin[b], m, cudaMemcpyHostToDevice, c->stream));
@@ -333,18 +333,17 @@ int array_info(const pic_ctx *c, int which, void **dptr, long long *n) {
     return PIC_OK;
 }
 
+// status, counts and the last diagnostics, in one copy
+const int kStateWords = 3 + PIC_NDIAG;
+
 int sync_status(pic_ctx *c) {
+    CK(cudaMemcpyAsync(c->h_state, c->d_state, kStateWords * sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    unsigned st = 0;
-    CK(cudaMemcpy(&st, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    const unsigned st = (unsigned)c->h_state[0];
     for (int k = 0; k < 2; ++k)
-        if (c->sp[k].d_count) {
-            long long n = 0;
-            CK(cudaMemcpy(&n, c->sp[k].d_count, sizeof(long long), cudaMemcpyDeviceToHost));
-            c->sp[k].n_host = n;
-        }
+        if (c->sp[k].d_count) c->sp[k].n_host = c->h_state[1 + k];
     if (st) {
-        CK(cudaMemset(c->d_status, 0, sizeof(unsigned)));
+        CK(cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream));
         if (st & ST_NAN) return fail(c, PIC_ENAN, "non-finite particle momentum or position (particle skipped)");
         if (st & ST_OOB) return fail(c, PIC_EOOB, "particle stencil outside the field buffers (particle skipped)");
         if (st & ST_CFL) return fail(c, PIC_EOOB, "particle moved a cell or more in one step (particle skipped)");
@@ -550,9 +549,14 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     int r = PIC_OK;
     for (int k = 0; k < 6 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->field[k], (size_t)c->g.fsz * rs);
     for (int k = 0; k < 5 && r == PIC_OK; ++k) r = dalloc(c, (char **)&c->ring[k], ((size_t)c->g.rsz * rs + 15) / 16 * 16);
-    r = r ? r : dalloc(c, &c->d_status, sizeof(unsigned));
+    r = r ? r : dalloc(c, &c->d_state, kStateWords * sizeof(long long));
+    c->d_status = (unsigned *)c->d_state;
+    c->d_diag = (double *)(c->d_state + 3);
+    if (r == PIC_OK && cudaHostAlloc((void **)&c->h_state, kStateWords * sizeof(long long), cudaHostAllocDefault) != cudaSuccess) {
+        c->h_state = nullptr;
+        r = fail(c, PIC_ENOMEM, "cudaHostAlloc");
+    }
     r = r ? r : dalloc(c, &c->d_scratch_ll, 16 * sizeof(long long));
-    r = r ? r : dalloc(c, &c->d_diag, PIC_NDIAG * sizeof(double));
     if (c->tile > 0) {
         c->sort_slots = sort_slots(c->nkeys);
         r = r ? r : dalloc(c, &c->d_hist, sort_hist_bytes(c));
@@ -566,7 +570,7 @@ int pic_create(const PicParams *pp, int device, pic_ctx **out) {
     }
     for (int k = 0; k < 6; ++k) cudaMemsetAsync(c->field[k], 0, (size_t)c->g.fsz * rs, c->stream);
     for (int k = 0; k < 5; ++k) cudaMemsetAsync(c->ring[k], 0, (size_t)c->g.rsz * rs, c->stream);
-    cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream);
+    cudaMemsetAsync(c->d_state, 0, kStateWords * sizeof(long long), c->stream);
     if (c->tile > 0) {
         cudaMemsetAsync(c->d_hist, 0, sort_hist_bytes(c), c->stream);
         cudaMemsetAsync(c->d_blocksums, 0, sort_sums_bytes(c), c->stream);
@@ -605,7 +609,8 @@ int pic_destroy(pic_ctx *c) {
         if (c->h_pin[b]) cudaFreeHost(c->h_pin[b]);
         if (c->pin_ev[b]) cudaEventDestroy(c->pin_ev[b]);
     }
-    void *ptrs[] = {c->d_status, c->d_gtab, c->d_profile, c->d_stage, c->d_scratch_ll, c->d_diag,
+    if (c->h_state) cudaFreeHost(c->h_state);
+    void *ptrs[] = {c->d_state, c->d_gtab, c->d_profile, c->d_stage, c->d_scratch_ll,
                     c->d_hist, c->d_blocksums, c->d_nstrag};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -640,7 +645,7 @@ int pic_upload_array(pic_ctx *c, int which, const double *host) {
         if (r) return r;
         launch_convert_array(c, d, c->d_stage, n, 1);
     }
-    CK(cudaStreamSynchronize(c->stream));
+    // the host's values are in the pinned buffer: nothing to wait for
     return launch_check(c, "pic_upload_array");
 }
 
@@ -650,7 +655,6 @@ int pic_download_array(pic_ctx *c, int which, double *host) {
     void *d;
     long long n;
     if (array_info(c, which, &d, &n) != PIC_OK) return fail(c, PIC_EINVAL, "bad array id");
-    int st = sync_status(c);
     if (!c->fp32) {
         int r = staged_d2h(c, host, d, (size_t)n * sizeof(double));
         if (r) return r;
@@ -661,8 +665,7 @@ int pic_download_array(pic_ctx *c, int which, double *host) {
         r = staged_d2h(c, host, c->d_stage, (size_t)n * sizeof(double));
         if (r) return r;
     }
-    CK(cudaStreamSynchronize(c->stream));
-    return st;
+    return sync_status(c);
 }
 
 int pic_upload_particles(pic_ctx *c, int kind, const void *records, int64_t n) {
@@ -1118,10 +1121,8 @@ int pic_diagnostics(pic_ctx *c, double *out, int n) {
     if (!c || !out || n < 1) return PIC_EINVAL;
     cudaSetDevice(c->device);
     launch_diagnostics(c, c->d_diag);
-    double tmp[PIC_NDIAG];
-    CK(cudaMemcpyAsync(tmp, c->d_diag, sizeof tmp, cudaMemcpyDeviceToHost, c->stream));
     int st = sync_status(c);
-    for (int i = 0; i < n && i < PIC_NDIAG; ++i) out[i] = tmp[i];
+    for (int i = 0; i < n && i < PIC_NDIAG; ++i) std::memcpy(out + i, c->h_state + 3 + i, sizeof(double));
     return st;
 }
 

@@ -136,7 +136,7 @@ struct VisSink {
 struct Species {
     int64_t cap = 0;
     int64_t n_host = 0;      // host copy of the count (upper bound between syncs)
-    long long *d_count = nullptr;
+    long long *d_count = nullptr;   // in pic_ctx::d_state
     int cur = 0;             // which position buffer is current
     PartArrays a;            // the particles
     PartArrays b;            // destination of the counting sort (same shapes)
@@ -209,7 +209,11 @@ struct pic_ctx {
     void *field[6] = {};   // ex ey ez bx by bz (double* or float*)
     void *ring[5] = {};    // jx jy jz rho0 rho1
     pic::Species sp[2];
-    unsigned *d_status = nullptr;
+    // status bits (the first word), the species' counts and the diagnostics, in
+    // one block: what the host reads back at a synchronisation, through its
+    // pinned copy
+    long long *d_state = nullptr, *h_state = nullptr;
+    unsigned *d_status = nullptr;        // = d_state
     double *d_gtab = nullptr;
     int gtab_n = 0;
     double *d_profile = nullptr;
@@ -218,13 +222,14 @@ struct pic_ctx {
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
     long long *d_scratch_ll = nullptr;   // small counters
-    double *d_diag = nullptr;
+    double *d_diag = nullptr;            // = d_state + 3
     // pinned host staging for particle uploads / downloads: two buffers of
     // kPinRecords records each, used alternately so that the host copy of
     // one chunk overlaps the DMA of the other
     void *h_pin[2] = {nullptr, nullptr};
     int64_t pin_records = 0;
     cudaEvent_t pin_ev[2] = {nullptr, nullptr};
+    int pin_next = 0;                    // buffer the next upload starts with
     // tiling / sorting
     int tile = 0;                        // tile edge in cells (or nodes) (0: global-memory kernel only)
     int ntile[3] = {0, 0, 0};
