@@ -280,25 +280,16 @@ __global__ void __launch_bounds__(256) scatter_kernel(const __grid_constant__ Sc
 // each tile is given a range of the list, in no particular order of the
 // tiles, then the entries are scattered.
 
-// FP64: below this fraction of a species away from home, the particles away
-// from home are pushed by the global-memory kernel instead.  On the
-// 256x128x128 thermal plasma (1.4 % away two pushes after a sort) the
-// visitor lists measured even at 2nd order and 4 % slower at 4th (a tile's
-// few visitors add a partial round of batches, and the FP64 kernel has the
-// longer rounds); on the laser run (6 % away, relativistic electrons) they
-// win.  FP32 uses them at any fraction (1.6 % faster at 2nd order, 2.6 % at
-// 4th on the thermal plasma).
-inline double visitor_min_fraction(const pic_ctx *c) { return c->fp32 ? 0.0 : 0.03; }
-
-__host__ __device__ inline bool visitor_lists_pay(unsigned long long entries, long long particles, double min_frac) {
-    return (double)entries >= min_frac * (double)particles;
-}
-
+// The lists are used however few particles are away from home (FP64 pushes
+// used them from 3 % on, when a tile's few visitors added a partial round to a
+// CTA that took the species one after the other).  Now, with 1.4 % away on the
+// thermal plasma, ms per step of the tile kernel and the global kernel for the
+// rest, lists against no lists: FP64 2nd order, 256 x 128 x 128 cells 10.52 +
+// 0.00 against 10.34 + 0.50; 4th order, 128 x 64 x 64 cells 4.26 against 4.01 +
+// 0.25; laser run 1.57 against 1.56 + 0.06.
 struct VisArgs {
     int ntiles;
-    double min_frac;
     struct One {
-        const long long *count;
         const int *raw;
         int *vis;
         uint2 *off;
@@ -334,7 +325,7 @@ __global__ void __launch_bounds__(1024) vis_ranges_kernel(const __grid_constant_
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         VisState &v = *a.vs;
         v.nvis = min((long long)v.nraw[a.par], a.cap);
-        v.valid_cur = v.valid_next[a.par] && visitor_lists_pay(v.nvis, *a.count, va.min_frac);
+        v.valid_cur = v.valid_next[a.par];
         v.nraw[a.par ^ 1] = 0ull;
         v.valid_next[a.par ^ 1] = 1u;
         *a.nstrag = 0ull;
@@ -357,13 +348,12 @@ __global__ void __launch_bounds__(256) vis_scatter_kernel(const __grid_constant_
 static void launch_vis_build(pic_ctx *c, int mask) {
     VisArgs va{};
     va.ntiles = c->ntile[0] * c->ntile[1] * c->ntile[2];
-    va.min_frac = visitor_min_fraction(c);
     unsigned ns = 0;
     long long n = 0;
     for (int k = 0; k < 2; ++k) {
         if (!((mask >> k) & 1)) continue;
         Species &s = c->sp[k];
-        va.s[ns++] = VisArgs::One{s.d_count, s.vraw, s.vis, s.vis_off, s.vis_cnt, s.vs, s.vis_par, s.vcap, c->d_nstrag + k};
+        va.s[ns++] = VisArgs::One{s.vraw, s.vis, s.vis_off, s.vis_cnt, s.vs, s.vis_par, s.vcap, c->d_nstrag + k};
         s.vis_par ^= 1;
         s.strag_zero = true;
         n = std::max<long long>(n, s.vcap);
@@ -832,13 +822,10 @@ int tile_order_stats(pic_ctx *c, int kind, long long (&out)[4]) {
         // the lists the next push will read: built from what the last push
         // recorded unless a full sort comes first
         VisState v{};
-        long long n = 0;
         if (cudaMemcpy(&v, s.vs, sizeof v, cudaMemcpyDeviceToHost) != cudaSuccess) return PIC_ECUDA;
-        if (cudaMemcpy(&n, s.d_count, sizeof n, cudaMemcpyDeviceToHost) != cudaSuccess) return PIC_ECUDA;
         const bool built = s.vis_built_for == s.pushes_since_sort;
         out[0] = built ? (long long)v.nvis : std::min<long long>((long long)v.nraw[s.vis_par], s.vcap);
-        out[1] = built ? v.valid_cur
-                       : (v.valid_next[s.vis_par] && visitor_lists_pay((unsigned long long)out[0], n, visitor_min_fraction(c)));
+        out[1] = built ? v.valid_cur : v.valid_next[s.vis_par];
     }
     if (c->d_nstrag) {
         unsigned long long ns[2] = {0, 0};
