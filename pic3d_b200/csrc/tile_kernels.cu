@@ -1,4 +1,6 @@
-// Tiled gather + push + deposit with shared-memory staging.
+// The sort and the visitor lists of every tiled context, and the tiled gather +
+// push + deposit over tiles of cells: tile edges other than the default one,
+// which has tiles of nodes (tile_node_kernels.cu, tile_mma_kernels.cu).
 //
 // Particles of each species are kept in counting-sort order by tile (T^3
 // cells), then by half-cell octant of the position (which side of the cell
@@ -528,7 +530,8 @@ static void prepare_push(pic_ctx *c, int mask) {
 // ---------------------------------------------------------------------------
 // the tile kernel
 
-// Threads per CTA of an ordinary step (the kernel's launch bounds ask for
+// (The figures here were taken at the default edge, when it had tiles of
+// cells.)  Threads per CTA of an ordinary step (the kernel's launch bounds ask for
 // two CTAs per SM at 256 threads, one at 512: 128 registers either way).
 // Two CTAs of 256 threads (128 registers) where the shared memory of two
 // fits: FP32 (measured 1.46x faster at 4th order than one CTA with more
@@ -543,30 +546,17 @@ static void prepare_push(pic_ctx *c, int mask) {
 template <typename real, int P>
 constexpr int tile_threads() { return sizeof(real) == 4 || P == 3 ? 256 : 512; }
 
-// TT: the tile edge as a compile-time constant (0: from the arguments).
-// With the edge known, every stride of the shared boxes is a constant and
-// the stencil addresses fold into instruction offsets.
 // NT: threads per CTA of this instantiation (512: one CTA per SM)
-template <typename real, int P, bool SPIN, int TT, int NT>
+template <typename real, int P, bool SPIN, int NT>
 __global__ void __launch_bounds__(NT, (NT >= 512 ? 1 : 2)) tile_push_kernel(TileArgs<real> ta) {
     constexpr int H = P / 2;
     constexpr int NL = limbs<real>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     real *sf = reinterpret_cast<real *>(smem_raw);
     const Geom &g = ta.sp[0].g;
-    const int T = TT > 0 ? TT : ta.t.T;
+    const int T = ta.t.T;
     const int GE = gather_extent<P>(T), DE = deposit_extent<P>(T);
-    int gsy, gsz, GS, dsy, dsz, DS;
-    if constexpr (TT > 0) {
-        constexpr int ge = gather_extent<P>(TT), de = deposit_extent<P>(TT);
-        constexpr int gy = padded_row(ge, TT), gz = padded_plane(ge, TT);
-        constexpr int dy = padded_row(de, TT), dz = padded_plane(de, TT);
-        gsy = gy; gsz = gz; GS = ge * gz;
-        dsy = dy; dsz = dz; DS = de * dz;
-    } else {
-        gsy = ta.t.gsy; gsz = ta.t.gsz; GS = ta.t.gsize;
-        dsy = ta.t.dsy; dsz = ta.t.dsz; DS = ta.t.dsize;
-    }
+    const int gsy = ta.t.gsy, gsz = ta.t.gsz, GS = ta.t.gsize, dsy = ta.t.dsy, dsz = ta.t.dsz, DS = ta.t.dsize;
     const int G2 = GE * GE, G3 = G2 * GE, D2 = DE * DE, D3 = D2 * DE;
     unsigned *sa = reinterpret_cast<unsigned *>(sf + 6 * GS);   // [component][limb][DS]
     // per warp, two slots of one batch of particle inputs, [word][lane],
@@ -803,13 +793,11 @@ static void tile_push_t(pic_ctx *c, int mask) {
     const bool wide = tile_launch_threads(c) != NT;
     if constexpr (sizeof(real) == 8 && NT != 512) {
         if (wide) {
-            if (c->tile == 4) launch(tile_push_kernel<real, P, SPIN, 4, 512>, 512);
-            else launch(tile_push_kernel<real, P, SPIN, 0, 512>, 512);
+            launch(tile_push_kernel<real, P, SPIN, 512>, 512);
             return;
         }
     }
-    if (c->tile == 4) launch(tile_push_kernel<real, P, SPIN, 4, NT>, NT);   // the default edge: strides as constants
-    else launch(tile_push_kernel<real, P, SPIN, 0, NT>, NT);
+    launch(tile_push_kernel<real, P, SPIN, NT>, NT);
 }
 
 // the counts pic_particle_order_stats reports (host side, synchronising)
