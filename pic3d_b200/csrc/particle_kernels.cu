@@ -233,16 +233,7 @@ __device__ __forceinline__ void current_cell(const RemoveArgs &r, const RemoveAr
     }
     const double v0[3] = {a.x[i], a.y[i], a.z[i]};
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        double v = v0[d];
-        if (r.g.per[d]) {
-            if (v < 0.0) v += r.g.n[d];
-            if (v > (double)r.g.n[d]) v -= r.g.n[d];
-        }
-        const double xc = v - (double)(1 - r.g.mem);
-        c[d] = xc >= 0.0 ? (int)xc - (r.g.mem - 1) : -1;
-        nd[d] = xc >= 0.0 ? (int)(xc + 0.5) - (r.g.mem - 1) : -1;
-    }
+    for (int d = 0; d < 3; ++d) bin_of(r.g, d, v0[d], c[d], nd[d]);
 }
 
 // the tile whose slice of the sorted arrays holds index i

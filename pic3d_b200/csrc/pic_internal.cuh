@@ -110,10 +110,11 @@ constexpr int kOctants = 8;
 // entries under one of two counters, chosen by the host's parity
 // (Species::vis_par); building the lists from them starts the other one.
 // valid_cur: the lists the running push reads name every particle that is
-// away from its home tile (else the push falls back to handing such particles
-// to the global kernel).  valid_next: the same for the entries the running
-// push appends; cleared when vraw overflows or when a particle lands outside
-// the tile grid on a periodic axis.
+// away from its home tile (else, and right after a sort, which builds none,
+// the push falls back to handing such particles to the global kernel).
+// valid_next: the same for the entries the running push appends; cleared when
+// vraw overflows or when a particle lands outside the tile grid on a periodic
+// axis.
 struct VisState {
     unsigned long long nraw[2];   // entries appended to vraw
     unsigned valid_next[2], valid_cur;

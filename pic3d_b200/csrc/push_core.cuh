@@ -503,6 +503,22 @@ __device__ __forceinline__ real part_real(const PartIn<real> &in, int k) {
     else return __uint_as_float(in.v[k]);
 }
 
+// Cell and primal index (node), in domain coordinates, of the FP64 position v
+// on axis d as decode_old will see them: the same wrap, the same sums, the
+// same roundings (-1 below the buffers).  Whatever bins a particle for its
+// next push takes them from here.  Formed in another way they differ for
+// some positions: of the double below 3.5, v - floor(v) is below 1/2 (node 3)
+// while v + (mem - 1) + 1/2 rounds up (node 4, another tile).
+__device__ __forceinline__ void bin_of(const Geom &g, int d, double v, int &cell, int &node) {
+    if (g.per[d]) {
+        if (v < 0.0) v += g.n[d];
+        if (v > (double)g.n[d]) v -= g.n[d];
+    }
+    const double xc = v - (double)(1 - g.mem);
+    cell = xc >= 0.0 ? (int)xc - (g.mem - 1) : -1;
+    node = xc >= 0.0 ? (int)(xc + 0.5) - (g.mem - 1) : -1;
+}
+
 template <typename real>
 __device__ __forceinline__ void decode_old(const PushArgs<real> &a, long long p, const PartIn<real> &in,
                                            OldPos<real> &o) {
@@ -667,17 +683,7 @@ __device__ __forceinline__ bool push_move(const PushArgs<real> &a, long long p, 
         a.y1[p] = xn[1];
         a.z1[p] = xn[2];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            // the wrap and truncation of decode_old
-            double v = xn[d];
-            if (g.per[d]) {
-                if (v < 0.0) v += g.n[d];
-                if (v > (double)g.n[d]) v -= g.n[d];
-            }
-            const double xc = v - (double)(1 - g.mem);
-            cnew[d] = xc >= 0.0 ? (int)xc - (g.mem - 1) : -1;
-            nnew[d] = xc >= 0.0 ? (int)(xc + 0.5) - (g.mem - 1) : -1;
-        }
+        for (int d = 0; d < 3; ++d) bin_of(g, d, xn[d], cnew[d], nnew[d]);
     } else {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {

@@ -39,49 +39,45 @@ static inline void padded_strides(int e, int T, int &sy, int &sz) {
     sz = padded_plane(e, T);
 }
 
-// Sort key of a particle in cell (cx, cy, cz) whose position in the cell
-// lies in half-cell octant `oct` (bit d set: offset >= 1/2 along axis d, so
-// its primal stencil index, its node, is the cell's plus one along d).
-// Tiles of cells: tile, then octant, then cell within the tile.  Tiles of
-// nodes: tile, then node within the tile, x fastest, so that consecutive
-// particles share the y and z of their stencils.
-__device__ __forceinline__ int tile_key(const TileGeom &t, const int (&cell)[3], int oct) {
+// Sort key of a particle.  Tiles of cells: tile, then half-cell octant `oct`
+// (bit d set: the particle's node is its cell's plus one along d), then cell
+// within the tile; `at` is the cell.  Tiles of nodes: tile, then node within
+// the tile, x fastest, so that consecutive particles share the y and z of
+// their stencils; `at` is the node.
+__device__ __forceinline__ int tile_key(const TileGeom &t, const int (&at)[3], int oct) {
     const int T = t.T;
     int q[3], l[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        const int c = cell[d] + (t.nodes ? (oct >> d) & 1 : 0);
-        q[d] = c / T;
-        l[d] = c - q[d] * T;
+        q[d] = at[d] / T;
+        l[d] = at[d] - q[d] * T;
     }
     const int tile = (q[2] * t.nt[1] + q[1]) * t.nt[0] + q[0];
     return ((t.nodes ? tile : tile * kOctants + oct) * T + l[2]) * T * T + l[1] * T + l[0];
 }
 
-// sort key of particle i (FP64: periodic wrap as the next push will apply
-// it; cell clamped into the domain)
+// Sort key of particle i: cell and node as the next push will decode them,
+// clamped to cells 0 .. n - 1, or nodes 0 .. n.
 __device__ __forceinline__ int particle_key(const Geom &g, const TileGeom &t, const CellPack &cp, int fp32,
                                             const double *x, const double *y, const double *z, const int *cell,
                                             const float *ox, const float *oy, const float *oz, long long i) {
-    int c[3], oct = 0;
+    int c[3], nd[3];
     if (fp32) {
         cp.unpack(cell[i], c[0], c[1], c[2]);
-        oct = (ox[i] >= 0.5f ? 1 : 0) | (oy[i] >= 0.5f ? 2 : 0) | (oz[i] >= 0.5f ? 4 : 0);
+        const float o[3] = {ox[i], oy[i], oz[i]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) nd[d] = c[d] + (o[d] >= 0.5f ? 1 : 0);
     } else {
-        double v[3] = {x[i], y[i], z[i]};
+        const double v[3] = {x[i], y[i], z[i]};
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            if (g.per[d]) {
-                if (v[d] < 0.0) v[d] += g.n[d];
-                if (v[d] > (double)g.n[d]) v[d] -= g.n[d];
-            }
-            const double f = floor(v[d]);
-            c[d] = (int)f;
-            oct |= (v[d] - f >= 0.5 ? 1 : 0) << d;
-        }
+        for (int d = 0; d < 3; ++d) bin_of(g, d, v[d], c[d], nd[d]);
     }
+    int oct = 0;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) c[d] = min(max(c[d], 0), g.n[d] - 1);
+    for (int d = 0; d < 3; ++d) {
+        oct |= (nd[d] > c[d] ? 1 : 0) << d;
+        c[d] = t.nodes ? min(max(nd[d], 0), g.n[d]) : min(max(c[d], 0), g.n[d] - 1);
+    }
     return tile_key(t, c, oct);
 }
 
@@ -162,8 +158,11 @@ __device__ __forceinline__ unsigned block_exclusive(unsigned s, unsigned &total)
 
 // Sums of the histogram's blocks of kSortKeysPerBlock keys; the last block to
 // finish turns them into exclusive offsets (sums[nb]: the total), so that the
-// scan takes two launches.  Every particle is at home after the sort: the
-// visitor lists are emptied, the straggler count too.
+// scan takes two launches.  The visitor lists and the straggler count are
+// emptied.  After the sort every particle is at home, except one whose cell was
+// clamped into the grid (x = n on a periodic axis where tiles hold cells, a
+// position outside the domain): no list names it, so the lists do not count
+// as valid for the push that follows and it goes to the global kernel.
 __global__ void __launch_bounds__(1024) sort_sums_kernel(const __grid_constant__ SortArgs sa, int nb) {
     const SortArgs::One &a = sa.s[blockIdx.y];
     __shared__ bool last;
@@ -202,7 +201,7 @@ __global__ void __launch_bounds__(1024) sort_sums_kernel(const __grid_constant__
         if (a.vs) {
             a.vs->nraw[a.par] = 0ull;
             a.vs->valid_next[a.par] = 1u;
-            a.vs->valid_cur = 1u;
+            a.vs->valid_cur = 0u;   // a home particle found away from its tile: the global kernel
             a.vs->total = 0u;
             a.vs->nvis = 0ull;
         }
