@@ -246,7 +246,9 @@ __global__ void __launch_bounds__(NodeTile2<real, RHO>::kThreads, NodeTile2<real
             // ---- the factors of the particles that keep their node ----------
             const bool moves = dep && (mv.i1[0] != mv.i2[0] || mv.i1[1] != mv.i2[1] || mv.i1[2] != mv.i2[2]);
             const bool sums = dep && !moves && (RHO || mv.moved);
-            // (every lane has read its inputs: the table takes their place)
+            // The table takes the place of the batch's inputs: every lane has read
+            // its own (the weight last) before another stores there.
+            __syncwarp();
             const unsigned changes = __ballot_sync(0xffffffffu, moves);
             real *tab = reinterpret_cast<real *>(slot ? wb + L::kSlot : wb);
             const int tab_at = (int)(tab - sf);
