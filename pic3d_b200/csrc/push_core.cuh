@@ -567,13 +567,16 @@ __device__ __forceinline__ void decode_old(const PushArgs<real> &a, long long p,
 }
 
 // 1 / sqrt(x), x >= 1: the library's FP64 function (1 ulp); in FP32 the
-// hardware approximation (2 ulp) with one Newton step (x = inf, where the
-// step is not a number, gives 0 as the division by gamma did).  A square root
-// and the divisions by it cost three times as many instructions.
+// hardware approximation (2 ulp) with one Newton step, whose residual
+// 1 - x y^2 is formed with the rounding of x y, so that the result is rounded
+// once (x = inf, where the step is not a number, gives 0 as the division by
+// gamma did).  A square root and the divisions by it cost three times as many
+// instructions; without the rounding of x y the FP32 moves were 1 % less
+// accurate than with them.
 __device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
 __device__ __forceinline__ float inv_sqrt(float x) {
-    const float y = rsqrtf(x);
-    return y > 0.0f ? fmaf(0.5f * y, fmaf(-x * y, y, 1.0f), y) : y;
+    const float y = rsqrtf(x), h = x * y, l = fmaf(x, y, -h);
+    return y > 0.0f ? fmaf(0.5f * y, fmaf(-l, y, fmaf(-h, y, 1.0f)), y) : y;
 }
 
 // A particle's move as its deposit needs it: old and new primal index, the
@@ -617,19 +620,20 @@ __device__ __forceinline__ bool push_move(const PushArgs<real> &a, long long p, 
     real b2 = gather<real, P, LDG>(fv[5], id[0] - H, id[1] - H, ip[2] - H, wd[0], wd[1], wp[2]);
     // Boris (particle.cpp:271-306)
     const real qm = a.qm;
-    real ex_p = e0 * qm, ey_p = e1 * qm, ez_p = e2 * qm;
-    real bx_p = b0 * qm, by_p = b1 * qm, bz_p = b2 * qm;
-    real px1 = pm.px[pm.i] + ex_p, py1 = pm.py[pm.i] + ey_p, pz1 = pm.pz[pm.i] + ez_p;
+    // The half kicks are fused multiply-adds by name: left to the compiler, the
+    // rounding of qm E enters twice or not at all, as its heuristics have it
+    // (FP32 momenta 34 % less accurate where it does).
+    const real px1 = fma(e0, qm, pm.px[pm.i]), py1 = fma(e1, qm, pm.py[pm.i]), pz1 = fma(e2, qm, pm.pz[pm.i]);
     const real ig1 = inv_sqrt(real(1) + (px1 * px1 + py1 * py1 + pz1 * pz1));
-    real tx = bx_p * ig1, ty = by_p * ig1, tz = bz_p * ig1;
+    real tx = b0 * qm * ig1, ty = b1 * qm * ig1, tz = b2 * qm * ig1;
     real tt = real(2) / (real(1) + tx * tx + ty * ty + tz * tz);
     real sx = tx * tt, sy = ty * tt, sz = tz * tt;
     real px2 = px1 + (py1 * tz - pz1 * ty);
     real py2 = py1 + (pz1 * tx - px1 * tz);
     real pz2 = pz1 + (px1 * ty - py1 * tx);
-    real pxn = px1 + (py2 * sz - pz2 * sy) + ex_p;
-    real pyn = py1 + (pz2 * sx - px2 * sz) + ey_p;
-    real pzn = pz1 + (px2 * sy - py2 * sx) + ez_p;
+    real pxn = fma(e0, qm, px1 + (py2 * sz - pz2 * sy));
+    real pyn = fma(e1, qm, py1 + (pz2 * sx - px2 * sz));
+    real pzn = fma(e2, qm, pz1 + (px2 * sy - py2 * sx));
     const real g2 = real(1) + (pxn * pxn + pyn * pyn + pzn * pzn);
     const real ig = inv_sqrt(g2);
     // move in cell units (particle.cpp:313-315)
