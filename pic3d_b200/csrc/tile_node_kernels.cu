@@ -51,9 +51,10 @@ struct NodeTile2 {
     // Accumulators: three neighbouring nodes' pairs of points {0, 1, 2} +
     // {0, 1, 2} dsy + {0, 1, 2} dsz, one bank shared.
     static constexpr int DE = T + 2 * H + 2, dsy = DE, dsz = DE * DE + 3, DS = DE * dsz;
-    // One particle's factors: 6 fluxes, charge, pad, then (s, d) of x, y, z;
-    // a stride that spreads the lanes' stores over the banks
-    static constexpr int TS = F64 ? 26 : 28;
+    // One particle's factors: 6 fluxes, charge, pad, then (s, d) of x, y, z,
+    // then (rho) the new shapes of z, a zero, those of x and y; a stride that
+    // spreads the lanes' stores over the banks
+    static constexpr int kPairs = 8, kNew = kPairs + 6 * P, TS = RHO ? 38 : F64 ? 26 : 28;
     static constexpr int KW = PartIn<real>::kWords;
     // CTAs of 4 warps, as many per SM as shared memory (FP64) or registers
     // (FP32) allow: the others cover one's staging, flush and last partial
@@ -75,20 +76,73 @@ struct NodeTile2 {
     static_assert(kCtas * (kBytes + 1024 + 128) <= 228 * 1024, "the CTAs of an SM share 228 KB");
 };
 
-// the sum of some particles' contributions to a point, scaled
-__device__ __forceinline__ void add_sum(unsigned *a, int lstride, double v) {
-    const long long q = __double2ll_rn(v);
-    atomicAdd(a, (unsigned)q & kLimbMask);
-    atomicAdd(a + lstride, (unsigned)(q >> kLimbBits) & kLimbMask);
-    atomicAdd(a + 2 * lstride, (unsigned)(int)(q >> (2 * kLimbBits)));
+// The sums over some particles (at most 32) of the contributions f w to two
+// points, in steps of the accumulators, and their addition to the points.
+// FP64: the steps are 2^-49 of the largest contribution, far above the
+// rounding of a sum in double.
+template <typename real>
+struct PairSum {
+    double v[2] = {0.0, 0.0};
+    __device__ __forceinline__ void add(Pair<double> f, double w0, double w1) {
+        v[0] = fma(f.s, w0, v[0]);
+        v[1] = fma(f.d, w1, v[1]);
+    }
+    template <int I>
+    __device__ __forceinline__ void to(unsigned *a, int lstride) const {
+        const long long q = __double2ll_rn(v[I]);
+        atomicAdd(a, (unsigned)q & kLimbMask);
+        atomicAdd(a + lstride, (unsigned)(q >> kLimbBits) & kLimbMask);
+        atomicAdd(a + 2 * lstride, (unsigned)(int)(q >> (2 * kLimbBits)));
+    }
+};
+
+// FP32: a sum in one register loses what the accumulators would have kept (64
+// particles per node, 0.3 c thermal: currents 12 % less accurate than with
+// an addition per particle).  It is kept in two: `hi` starts at 1.5 2^41, where
+// a float's last bit is 2^18 (one step of the upper limb), so that it takes
+// the multiple of 2^18 nearest to each contribution (up to 2^31), without
+// error; `lo` takes the rest, up to 2^17 each, rounded to a fraction of a step.
+// Two points per instruction (FP32 pairs).  128 x 64 x 64 cells, 8 + 8 particles
+// per cell: 848 us against 796 with one register; sums in FP64, whose operands
+// have to be converted, 893, two registers without pairs 881.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
-__device__ __forceinline__ void add_sum(unsigned *a, int lstride, float v) {
-    // up to 32 times a particle's 2^31: split before the conversion
-    const int hi = __float2int_rd(v * (1.0f / (1 << kLimbBits)));
-    const unsigned lo = __float2uint_rn(fmaf((float)hi, -(float)(1 << kLimbBits), v));
-    atomicAdd(a, lo);
-    atomicAdd(a + lstride, (unsigned)hi);
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+template <>
+struct PairSum<float> {
+    static constexpr float kStart = 3298534883328.0f;
+    unsigned long long hi = pack2(kStart, kStart), lo = 0ull;
+    __device__ __forceinline__ void add(Pair<float> f, float w0, float w1) {
+        const unsigned long long ff = pack2(f.s, f.d), ww = pack2(w0, w1), t = fma2(ff, ww, hi);
+        lo = add2(lo, fma2(ff, ww, sub2(hi, t)));   // f w - (t - hi)
+        hi = t;
+    }
+    template <int I>
+    __device__ __forceinline__ void to(unsigned *a, int lstride) const {
+        static_assert(kLimbBits == 18, "the last bit of hi is one step of the upper limb");
+        const int upper = (int)(unsigned)(hi >> (32 * I)) - __float_as_int(kStart);
+        const int rest = __float2int_rn(__uint_as_float((unsigned)(lo >> (32 * I))));
+        atomicAdd(a, (unsigned)rest & kLimbMask);
+        atomicAdd(a + lstride, (unsigned)(upper + (rest >> kLimbBits)));
+    }
+};
 
 template <typename real, bool SPIN, bool RHO>
 __global__ void __launch_bounds__(NodeTile2<real, RHO>::kThreads, NodeTile2<real, RHO>::kCtas)
@@ -256,31 +310,33 @@ __global__ void __launch_bounds__(NodeTile2<real, RHO>::kThreads, NodeTile2<real
             if (sums) {
                 node = (mv.i1[0] - lo[0]) + T * ((mv.i1[1] - lo[1]) + T * (mv.i1[2] - lo[2]));
                 real *row = tab + lane * L::TS;
-                real f[8];
+                Pair<real> f[4];   // (x, y) of the first flux, of the second, z, charge
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    real w0[P], ds[P];
+                    real w0[P], ds[P], w1[P];
                     shape_weights(mv.d0[d], w0);
                     if constexpr (sizeof(real) == 8) {
-                        real w1[P];
                         shape_weights(mv.dm[d], w1);
 #pragma unroll
                         for (int q = 0; q < P; ++q) ds[q] = w1[q] - w0[q];
                     } else {
                         shape_diff(mv.d0[d], mv.dm[d], ds);
+                        if constexpr (RHO) shape_weights(mv.d0[d] + mv.dm[d], w1);
                     }
                     const real q0 = -(mv.qw * a.d_dt[d] * ta.scale[d]);
-                    f[2 * d] = q0 * ds[0];
-                    f[2 * d + 1] = q0 * (ds[0] + ds[1]);
+                    (d == 0 ? f[0].s : d == 1 ? f[0].d : f[2].s) = q0 * ds[0];
+                    (d == 0 ? f[1].s : d == 1 ? f[1].d : f[2].d) = q0 * (ds[0] + ds[1]);
 #pragma unroll
-                    for (int q = 0; q < P; ++q)
-                        reinterpret_cast<Pair<real> *>(row + 8)[3 * d + q] =
+                    for (int q = 0; q < P; ++q) {
+                        reinterpret_cast<Pair<real> *>(row + L::kPairs)[3 * d + q] =
                             Pair<real>{w0[q] + real(0.5) * ds[q], ds[q] * real(0.28867513459481287)};
+                        if constexpr (RHO) row[L::kNew + (d == 2 ? 0 : 4 + 3 * d) + q] = w1[q];
+                    }
                 }
-                f[6] = RHO ? mv.qw * ta.scale[3] : real(0);
-                f[7] = real(0);
+                if constexpr (RHO) row[L::kNew + 3] = real(0);
+                f[3] = Pair<real>{RHO ? mv.qw * ta.scale[3] : real(0), real(0)};
 #pragma unroll
-                for (int q = 0; q < 8; q += 2) *reinterpret_cast<Pair<real> *>(row + q) = Pair<real>{f[q], f[q + 1]};
+                for (int q = 0; q < 4; ++q) reinterpret_cast<Pair<real> *>(row)[q] = f[q];
             }
             if (moves) queue[queued + __popc(changes & ((1u << lane) - 1u))] = loc.x | (k << 31);
             queued += __popc(changes);
@@ -306,51 +362,44 @@ __global__ void __launch_bounds__(NodeTile2<real, RHO>::kThreads, NodeTile2<real
                         at = nd;
                     }
                 }
-                real j[6], r[RHO ? 3 : 1];
-#pragma unroll
-                for (int q = 0; q < 6; ++q) j[q] = real(0);
-                if constexpr (RHO) r[0] = r[1] = r[2] = real(0);
+                // (jx, jy) of the first points, of the second, (jz, jz); rho
+                PairSum<real> j[3], r[RHO ? 2 : 1];
                 // lanes whose node has no more particles read zeros (their last
                 // row again, with zeros for its fluxes only: 2 % slower)
 #pragma unroll 2
                 for (int it = 0; it < n; ++it) {
                     const real *row = sf + (todo ? tab_at + (__ffs(todo) - 1) * L::TS : zero_at);
                     todo &= todo - 1;
-                    const Pair<real> *xyz = reinterpret_cast<const Pair<real> *>(row + 8);
+                    const Pair<real> *fl = reinterpret_cast<const Pair<real> *>(row),
+                                     *xyz = reinterpret_cast<const Pair<real> *>(row + L::kPairs);
                     const Pair<real> xu = xyz[u], yu = xyz[3 + u], yv = xyz[3 + v], zv = xyz[6 + v];
-                    const Pair<real> fx = *reinterpret_cast<const Pair<real> *>(row),
-                                     fy = *reinterpret_cast<const Pair<real> *>(row + 2),
-                                     fz = *reinterpret_cast<const Pair<real> *>(row + 4);
                     const real wx = yu.s * zv.s + yu.d * zv.d, wy = xu.s * zv.s + xu.d * zv.d,
                                wz = xu.s * yv.s + xu.d * yv.d;
-                    j[0] += fx.s * wx;
-                    j[1] += fx.d * wx;
-                    j[2] += fy.s * wy;
-                    j[3] += fy.d * wy;
-                    j[4] += fz.s * wz;
-                    j[5] += fz.d * wz;
+                    j[0].add(fl[0], wx, wy);
+                    j[1].add(fl[1], wx, wy);
+                    j[2].add(fl[2], wz, wz);
                     if constexpr (RHO) {
-                        // the new shapes: s + sqrt(3) d
-                        const real s3 = real(1.7320508075688772);
-                        const real w = row[6] * ((xu.s + s3 * xu.d) * (yv.s + s3 * yv.d));
-#pragma unroll
-                        for (int e = 0; e < 3; ++e) r[e] += w * (xyz[6 + e].s + s3 * xyz[6 + e].d);
+                        const real w = row[6] * (row[L::kNew + 4 + u] * row[L::kNew + 7 + v]);
+                        const Pair<real> *z = reinterpret_cast<const Pair<real> *>(row + L::kNew);
+                        r[0].add(z[0], w, w);
+                        r[1].add(z[1], w, w);
                     }
                 }
                 if (mine >= 0) {
                     unsigned *q0 = sa + ((at & 3) + 1) + (((at >> 2) & 3) + 1) * L::dsy + ((at >> 4) + 1) * L::dsz;
                     unsigned *qx = q0 + u * L::dsy + v * L::dsz, *qy = q0 + NL * L::DS + u + v * L::dsz,
                              *qz = q0 + 2 * NL * L::DS + u + v * L::dsy;
-                    add_sum(qx, L::DS, j[0]);
-                    add_sum(qx + 1, L::DS, j[1]);
-                    add_sum(qy, L::DS, j[2]);
-                    add_sum(qy + L::dsy, L::DS, j[3]);
-                    add_sum(qz, L::DS, j[4]);
-                    add_sum(qz + L::dsz, L::DS, j[5]);
+                    j[0].template to<0>(qx, L::DS);
+                    j[1].template to<0>(qx + 1, L::DS);
+                    j[0].template to<1>(qy, L::DS);
+                    j[1].template to<1>(qy + L::dsy, L::DS);
+                    j[2].template to<0>(qz, L::DS);
+                    j[2].template to<1>(qz + L::dsz, L::DS);
                     if constexpr (RHO) {
                         unsigned *qr = q0 + (3 + k) * NL * L::DS + u + v * L::dsy;
-#pragma unroll
-                        for (int e = 0; e < 3; ++e) add_sum(qr + e * L::dsz, L::DS, r[e]);
+                        r[0].template to<0>(qr, L::DS);
+                        r[0].template to<1>(qr + L::dsz, L::DS);
+                        r[1].template to<0>(qr + 2 * L::dsz, L::DS);
                     }
                 }
             }
