@@ -211,9 +211,10 @@ struct pic_ctx {
     void *ring[5] = {};    // jx jy jz rho0 rho1
     pic::Species sp[2];
     // status bits (the first word), the species' counts and the diagnostics, in
-    // one block: what the host reads back at a synchronisation, through its
-    // pinned copy
-    long long *d_state = nullptr, *h_state = nullptr;
+    // one block: what the host reads back at a synchronisation, through
+    // pinned memory once there is some (pin_state, in h_pin[0])
+    long long *d_state = nullptr, *pin_state = nullptr;
+    long long h_state[3 + PIC_NDIAG] = {};
     unsigned *d_status = nullptr;        // = d_state
     double *d_gtab = nullptr;
     int gtab_n = 0;
