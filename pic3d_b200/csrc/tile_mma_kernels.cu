@@ -230,7 +230,9 @@ __global__ void __launch_bounds__(NodeTile<real, P>::kThreads, NodeTile<real, P>
 
         // ---- push, one particle per lane ------------------------------------
         bool dep = false;      // the particle deposits
-        int row = -1;          // its row (y + 4 z of the node) if it takes part in the matrix products
+        // its row (y + 4 z of the node) if it takes part in the matrix products,
+        // -2: at rest, it adds no current
+        int row = -1;
         int geo = 0;           // lower node + 1 per axis (3 bits each), move in nodes + 1 per axis (2 bits each)
         Moved<real> mv;
         // (adjoint contexts: removed particles stay, dead)
@@ -265,7 +267,13 @@ __global__ void __launch_bounds__(NodeTile<real, P>::kThreads, NodeTile<real, P>
                         mn[d] = min(mv.i1[d], mv.i2[d]) - lo[d];
                         geo |= (mn[d] + 1) << (3 * d) | (cr[d] + 1) << (9 + 2 * d);
                     }
-                    if (cr[1] == 0 && cr[2] == 0 && mn[0] >= 0 && mn[0] + abs(cr[0]) < T) row = mn[1] + T * mn[2];
+                    // at rest (as Moved::moved, which costs FP64 2 % here): dm is
+                    // the new offset (FP64) or the move (FP32)
+                    bool rest = !RHO && cr[0] == 0 && cr[1] == 0 && cr[2] == 0;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) rest = rest && mv.dm[d] == (L::F64 ? mv.d0[d] : real(0));
+                    if (rest) row = -2;
+                    else if (cr[1] == 0 && cr[2] == 0 && mn[0] >= 0 && mn[0] + abs(cr[0]) < T) row = mn[1] + T * mn[2];
                 }
             } else if (!inside && i < mh[k] && vvalid[k]) {
                 // away from home: pushed from the visitor list of the tile it is in
@@ -297,7 +305,7 @@ __global__ void __launch_bounds__(NodeTile<real, P>::kThreads, NodeTile<real, P>
         // a Jy row (v < P), else the y point v - P of a Jz row.
         auto yz_row = [](int t, int n) { return 2 * t + (n >> 2); };
         unsigned reg = __ballot_sync(0xffffffffu, row >= 0);      // not yet summed
-        const unsigned irr = __ballot_sync(0xffffffffu, dep && row < 0);
+        const unsigned irr = __ballot_sync(0xffffffffu, dep && row == -1);
         unsigned todo = 0, sc = 0;   // of the current group of 8: to sum, to scatter
         int cur = -1, grp = -1;
 #pragma unroll 1

@@ -54,7 +54,7 @@ struct NodeTile2 {
     // One particle's factors: 6 fluxes, charge, pad, then (s, d) of x, y, z,
     // then (rho) the new shapes of z, a zero, those of x and y; a stride that
     // spreads the lanes' stores over the banks
-    static constexpr int kPairs = 8, kNew = kPairs + 6 * P, TS = RHO ? 38 : F64 ? 26 : 28;
+    static constexpr int kPairs = 8, kNew = kPairs + 6 * P, TS = RHO ? kNew + 12 : F64 ? kNew : kNew + 2;
     static constexpr int KW = PartIn<real>::kWords;
     // CTAs of 4 warps, as many per SM as shared memory (FP64) or registers
     // (FP32) allow: the others cover one's staging, flush and last partial

@@ -3,8 +3,9 @@
 Every particle has a weight of its own, far from its neighbours', so that a
 particle deposited with another's weight, or with inputs that were overwritten
 before it read them, shows at once.  Nodes hold none to several batches of
-particles; one step against the oracle at the one-step parity bounds (relative
-L2 1e-10 in FP64, 1e-5 in FP32).
+particles, all moving or half of them at rest (those add rho, no current); one
+step against the oracle at the one-step parity bounds (relative L2 1e-10 in
+FP64, 1e-5 in FP32).
 """
 import numpy as np
 import pytest
@@ -38,3 +39,25 @@ def test_every_particle_deposits_its_own_weight(ppc, mem, precision):
         bad = {k: v for k, v in errs.items() if v > tol}
         assert not bad, (n + 1, bad)
     sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("mem", [2, 4], ids=["o2", "o4"])
+@pytest.mark.parametrize("steps", [1, 2], ids=["rho", "no_rho_first"])
+def test_particles_at_rest_among_moving_ones(steps, mem, precision):
+    from pic3d_b200.simulation import Simulation
+    w = W.Workload(name="rest", nx=12, ny=10, nz=11, mem=mem, period=(1, 1, 1), ppc=(6, 0), u_th=(0.2, 0.0), steps=steps)
+    parts = W.make_particles(w, seed=9)
+    still = np.random.default_rng(1).random(len(parts[0])) < 0.5
+    for f in ("px", "py", "pz"):
+        parts[0][f][still] = 0.0
+    parts[0]["gamma"] = np.sqrt(1.0 + parts[0]["px"] ** 2 + parts[0]["py"] ** 2 + parts[0]["pz"] ** 2)
+    o = O.Oracle(w, parts)
+    for s in range(1, steps + 1):
+        o.step(s)
+    sim = Simulation(w, precision=precision)
+    sim.upload_particles(0, parts[0])
+    sim.run_main_time_loop(steps)
+    errs = array_errors(sim.state(), o.state())
+    sim.close()
+    assert max(errs.values()) < (TOL_FP64 if precision == "fp64" else TOL_FP32), errs
