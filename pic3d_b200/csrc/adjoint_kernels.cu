@@ -556,9 +556,8 @@ __global__ void __launch_bounds__(128) adj_push_kernel(AdjPushArgs<real> a) {
 //      adjoints of its gathered E and B (six values) and their largest
 //      magnitude per component;
 //   3. adds every particle's field adjoint times its gather weights into
-//      fixed-point shared accumulators (20-bit limbs as the forward deposit,
-//      scaled so that the largest value fits), then flushes them with one
-//      pass of global atomics.
+//      fixed-point shared accumulators (20-bit limbs, scaled so that the
+//      largest value fits), then flushes them with one pass of global atomics.
 // Particles that left their tile since the sort go to the global kernel
 // afterwards.
 //
@@ -987,7 +986,6 @@ __global__ void adj_seed_kinetic_kernel(Geom g, CellPack cp, int fp32, long long
 
 }  // namespace pic
 
-// moves of per-particle arrays between orders (bit copies)
 // Several device arrays of 16-byte aligned addresses copied in one launch
 // (blockIdx.y: the array).  A tape slot has 16 or more of them and is saved
 // before every push: one by one, 1.9 us and a launch each, they took a tenth
@@ -1010,7 +1008,8 @@ __global__ void __launch_bounds__(256) copy_arrays_kernel(const __grid_constant_
         ((unsigned char *)dst)[words * 16 + threadIdx.x] = ((const unsigned char *)src)[words * 16 + threadIdx.x];
 }
 
-// The same permutation of several per-particle arrays in one launch:
+// The same permutation of several per-particle arrays in one launch (bit
+// copies between orders):
 // out[map[i]] = in[i], or (GATHER) out[i] = in[map[i]].
 struct PermuteList {
     const unsigned long long *ds[8];

@@ -286,10 +286,12 @@ __device__ __forceinline__ void atomic_add(float *p, float v) { atomicAdd(p, v);
 //              (NL = 2 limbs for FP32, 3 for FP64).  Integer sums do not
 //              depend on the order of the additions.  (Shared-memory 64-bit
 //              integer atomics measured 2.6x slower on the whole kernel.)
-// One contribution stays below 2^kFixedBits (31 FP32, 49 FP64), so that
-// 16383 additions per point fit: the unsigned 18-bit limb sums in 32 bits,
-// the signed top limb sums (below 2^13 resp. 2^15 each) in 32 bits, and
-// the reassembled total in 64 bits.
+// One particle's contribution to a point stays below 2^fixed_bits (31 FP32, 49
+// FP64), and a tile that takes this path holds at most 16383 particles.  However
+// they are grouped (an addition may stand for the sum of up to 32 of them), a
+// point's total stays below 2^63 (FP64), the signed top limb, its multiple of
+// 2^36 (FP64) or 2^18 (FP32), below 2^28; and at most 16383 additions of less
+// than 2^18 each go to a lower, unsigned limb, which stays below 2^32.
 constexpr int kLimbBits = 18;
 constexpr unsigned kLimbMask = (1u << kLimbBits) - 1u;
 template <typename real>

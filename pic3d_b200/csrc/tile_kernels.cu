@@ -10,10 +10,11 @@
 //      (T + 2H + 1 points per axis) in shared memory,
 //   2. clears shared-memory accumulators for jx, jy, jz, rho0, rho1 over the
 //      deposit footprint (T + 2H + 3 points per axis),
-//   3. pushes the particles whose sort key falls in the tile, both species,
-//      gathering from and depositing into shared memory; a particle that has
-//      left the tile since the last sort takes the global-memory path in the
-//      same loop (read-only loads, global atomics),
+//   3. pushes the tile's particles, both species, gathering from and
+//      depositing into shared memory: those whose sort key fell in it and that
+//      are still in it, and its visitor list, which names those that have come
+//      into it since the sort (without valid lists a particle away from home is
+//      left to the global kernel, which runs after this one),
 //   4. flushes the accumulators with one coalesced pass of global atomics
 //      (zero entries skipped); halos of neighbouring tiles overlap, hence the
 //      atomics.

@@ -21,9 +21,9 @@
 // (C the running sum of ds along the component's axis), i.e. matrix products
 // whose inner dimension is the particle.  A warp forms them with FP64
 // m8n8k4 matrix instructions, four particles per instruction, in both
-// precisions (FP32 has no matrix unit of its own accuracy; the products and
-// sums of its FP32 factors are then exact), and adds each row's sum to the
-// shared accumulators once.  The scatter by particle this replaces spent
+// precisions (FP32 has no matrix unit of its own accuracy; the products of its
+// FP32 factors are then exact, their sums rounded at 53 bits), and adds each
+// row's sum to the shared accumulators once.  The scatter by particle this replaces spent
 // 300 x 3 (FP64) shared atomics per particle, 3.2 cycles of the shared-memory
 // pipe for each warp's worth.
 // Particles that change their y or z node, leave the row's eight columns, or
