@@ -546,7 +546,8 @@ void node_tile_push(pic_ctx *c, int mask) {
 // Tiles of nodes: both orders at the default tile edge.  The matrix deposit
 // here is for 4th order; measured per launch on 128 x 64 x 64 cells, 8 + 8
 // particles per cell (tiles of cells with a scatter per particle first): FP64
-// 7.08 -> 4.07 ms, FP32 3.72 -> 2.42 ms.  At 2nd order the factors of its
+// 7.08 -> 4.07 ms, FP32 3.72 -> 2.42 ms (in FP64 without the 1.4 % away from
+// home, now in the tiles' lists: 0.25 ms).  At 2nd order the factors of its
 // products cost more to make (FP32 1.23 ms) than a particle's 54 points to
 // scatter (1.01 ms): tile_node_kernels.cu sums them per node instead.  Other
 // edges keep the tiles of cells of tile_kernels.cu.

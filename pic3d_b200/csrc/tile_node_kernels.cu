@@ -20,8 +20,8 @@
 // address, and sorted so that they do not, the gather's loads conflict.  Node
 // order makes the gather's loads broadcasts and leaves 12 (18) atomics per
 // lane, node and batch.
-// What bounds it (128 x 64 x 64 cells, 8 + 8 per cell): in FP32 issue (63 % of
-// the slots) and the shared-memory pipe (80 %) together, 795 us against 993 us
+// What bounds it (128 x 64 x 64 cells, 8 + 8 per cell): in FP32 issue (65 % of
+// the slots) and the shared-memory pipe (75 %) together, 850 us against 993 us
 // with the scatter; in FP64 the shared-memory pipe (83 %), on 256 x 128 x 128
 // cells 10.3 against 11.5 ms, with rho 13.5 against 17.0 ms.  About half of the
 // pipe's time goes to the gather's 162 loads.
@@ -103,7 +103,7 @@ struct PairSum {
 // the multiple of 2^18 nearest to each contribution (up to 2^31), without
 // error; `lo` takes the rest, up to 2^17 each, rounded to a fraction of a step.
 // Two points per instruction (FP32 pairs).  128 x 64 x 64 cells, 8 + 8 particles
-// per cell: 848 us against 796 with one register; sums in FP64, whose operands
+// per cell: 850 us against 796 with one register; sums in FP64, whose operands
 // have to be converted, 893, two registers without pairs 881.
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
     unsigned long long r;
